@@ -4,8 +4,9 @@
 //     global-colouring executor (problem.hpp:90-194, one launch and one
 //     cudaDeviceSynchronize per colour).  One launch per iteration, one thread
 //     per cell, mapping rows read as vectors, read sets gathered straight from
-//     HBM/L2, increments added with native atomics (f64 RED; one 16-byte f32x4
-//     RED per row for the FP32 loop).  With warp aggregation, lanes whose
+//     HBM/L2, increments added with native atomics (f64 RED, AOS rows laid end
+//     to end across the warp first; one 16-byte f32x4 RED per row for the FP32
+//     loop).  With warp aggregation, lanes whose
 //     slot targets the same point are grouped with __match_any_sync and summed
 //     in registers by a segmented shuffle tree before one lane issues the
 //     atomics.
@@ -177,7 +178,42 @@ __device__ __forceinline__ void load_row(const uint32_t *__restrict__ map, uint3
 // (a) atomic executor
 // ===========================================================================
 
+constexpr uint32_t kAtomicWarps = 8;  // warps per CTA of the atomic kernels
+
 template <class T> __device__ __forceinline__ void atomic_add(T *a, T v) { atomicAdd(a, v); }
+
+// Add the warp's 32 rows of K doubles (row of lane l: inc, for point key,
+// kNoPoint: none) to AOS point data, through the warp's slice of shared
+// memory: reduction instruction i then covers elements [32 i, 32 i + 32) of
+// the rows laid end to end, so that neighbouring lanes fall into the same
+// 32-byte sectors of `out` (K = 4: 8 whole sectors an instruction).  Lane by
+// lane, component by component, each instruction touched 32 sectors, and the
+// L2's rate of atomic sectors bounded the loop: res_calc 1000^2 (4 doubles a
+// row) after RCM 97.3 us then, 45.1 us now; getacc 1024^2 108.0 and 45.5 us;
+// LULESH 96^3 (3 doubles) 92.5 and 49.6 us.  FP32 rows of 4 are one 16-byte
+// reduction and SOA data one run of addresses a component: neither needs it.
+constexpr uint32_t kNoPoint = 0xFFFFFFFFu;
+template <int K>
+__device__ __forceinline__ void add_rows_f64(double *__restrict__ out, double *buf, uint32_t key,
+                                             const double (&inc)[K]) {
+  const uint32_t lane = threadIdx.x & 31u;
+  __syncwarp();  // the previous slot's rows have been read
+  if constexpr (K % 2 == 0) {
+#pragma unroll
+    for (int k = 0; k < K; k += 2)
+      *reinterpret_cast<double2 *>(buf + lane * K + k) = make_double2(inc[k], inc[k + 1]);
+  } else {
+#pragma unroll
+    for (int k = 0; k < K; ++k) buf[lane * K + k] = inc[k];
+  }
+  __syncwarp();
+#pragma unroll
+  for (int i = 0; i < K; ++i) {
+    const uint32_t e = i * 32u + lane, row = e / K;
+    const uint32_t p = __shfl_sync(0xFFFFFFFFu, key, row);
+    if (p != kNoPoint) atomic_add(out + (size_t)p * K + (e - row * K), buf[e]);
+  }
+}
 
 // Cells [base, base + 32) of one mesh, one per lane of the calling warp
 // (cells past n_cells are masked): compute, optionally aggregate by target
@@ -212,7 +248,7 @@ __device__ __forceinline__ void atomic_warp(const LoopData &d, uint32_t base) {
   }
 #pragma unroll
   for (int s = 0; s < D; ++s) {
-    const uint32_t key = valid ? rows.p[0][s] : 0xFFFFFFFFu;
+    const uint32_t key = valid ? rows.p[0][s] : kNoPoint;
     bool leader = valid;
     if constexpr (AGG) {
       const unsigned peers = __match_any_sync(0xFFFFFFFFu, key);
@@ -232,7 +268,10 @@ __device__ __forceinline__ void atomic_warp(const LoopData &d, uint32_t base) {
       }
       leader = valid && rank == 0;
     }
-    if (leader) {
+    if constexpr (!SOA && sizeof(out_t) == 8) {
+      __shared__ __align__(16) out_t s_rows[kAtomicWarps][32 * K];
+      add_rows_f64<K>(out, s_rows[threadIdx.x >> 5], leader ? key : kNoPoint, inc[s]);
+    } else if (leader) {
       if constexpr (!SOA && sizeof(out_t) == 4 && K == 4) {
         float4 v = make_float4(inc[s][0], inc[s][1], inc[s][2], inc[s][3]);
         atomicAdd(reinterpret_cast<float4 *>(out) + key, v);

@@ -1,0 +1,45 @@
+"""The atomic executor's reductions on the GPU: rows of every width laid out
+across warps of every fill.  Tolerances as for every atomic run: 1e-12 (FP64)
+and 1e-5 (FP32) normwise against the oracle's serial loop."""
+import numpy as np
+import pytest
+
+from cuda_fot_b200 import meshgen as mg
+from oracle import oracle_py as O
+from tests.helpers import rel_err
+
+pytestmark = pytest.mark.gpu
+
+
+def F():
+    from cuda_fot_b200 import fot
+    return fot
+
+
+def cut(md, n):
+    """The mesh's first n cells (all points stay)."""
+    md.n_cells = n
+    md.maps = [np.ascontiguousarray(m[:n]) for m in md.maps]
+    md.cell_data = [np.ascontiguousarray(d[:, :n]) for d in md.cell_data]
+    return md
+
+
+MESHES = {"res_calc": lambda lay: mg.res_calc(24, 20, 5, lay), "mini_aero": lambda lay: mg.mini_aero(8, 5, lay),
+          "lulesh": lambda lay: mg.lulesh(9, 5, lay), "volna": lambda lay: mg.volna(20, 16, 5, lay),
+          "getacc": lambda lay: mg.getacc(30, 22, 5, lay)}
+
+
+def check(md, flags, iters=2):
+    p = F().Problem.from_mesh(md)
+    plan = p.plan(F().EXEC_ATOMIC, 256, flags)
+    plan.run(iters)
+    p.sync()
+    assert rel_err(p.point_weights(0), O.serial(md, iters)[0][0]) <= (1e-5 if md.loop == mg.VOLNA else 1e-12)
+
+
+@pytest.mark.parametrize("flags", [0, 1])
+@pytest.mark.parametrize("layout", ["aos", "soa"])
+@pytest.mark.parametrize("n", [1, 31, 32, 33, 255, 257, 600])
+@pytest.mark.parametrize("name", list(MESHES))
+def test_rows_of_partly_filled_warps(name, n, layout, flags):
+    check(cut(MESHES[name](layout), n), flags)
