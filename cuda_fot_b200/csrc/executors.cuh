@@ -6,10 +6,9 @@
 //     per cell, mapping rows read as vectors, read sets gathered straight from
 //     HBM/L2, increments added with native atomics (f64 RED, AOS rows laid end
 //     to end across the warp first; one 16-byte f32x4 RED per row for the FP32
-//     loop).  With warp aggregation, lanes whose
-//     slot targets the same point are grouped with __match_any_sync and summed
-//     in registers by a segmented shuffle tree before one lane issues the
-//     atomics.
+//     loop).  With warp aggregation, runs of neighbouring lanes whose
+//     slot targets one point are summed in registers by a segmented shuffle
+//     tree before the run's first lane issues the atomics.
 //
 // (b) Hierarchical colouring (FOT_EXEC_HIER / _HIER_LAUNCH) -- replaces
 //     loopGPUHierarchical (problem.hpp:198-339) and its kernels
@@ -215,9 +214,34 @@ __device__ __forceinline__ void add_rows_f64(double *__restrict__ out, double *b
   }
 }
 
+// Warp aggregation: sum the rows of each run of neighbouring lanes with one
+// key into the run's first lane (returns true there).  Orderings sort cells by
+// their points, so that equal keys lie side by side (2 edges, 3 faces of a
+// first cell); equal keys further apart stay separate reductions.  A warp
+// without runs pays one shuffle and one vote.  Grouping every lane with
+// __match_any_sync instead and gathering the group lane by lane cost more than
+// the reductions it saved: volna 1024^2 72.4 us, 42.5 us by runs; res_calc
+// 1000^2 SOA 49.0 and 41.3 us; LULESH 96^3 SOA 74.2 and 45.7 us (after RCM).
+template <int K, class T>
+__device__ __forceinline__ bool sum_runs(uint32_t key, T (&inc)[K]) {
+  const uint32_t lane = threadIdx.x & 31u;
+  const uint32_t before = __shfl_up_sync(0xFFFFFFFFu, key, 1);
+  const unsigned first = __ballot_sync(0xFFFFFFFFu, lane == 0 || before != key);
+  // bit l: lane l + off lies in lane l's run (the same mask in every lane)
+  unsigned inside = ~first >> 1;
+  for (uint32_t off = 1; inside; inside &= inside >> off, off <<= 1) {
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+      const T v = __shfl_down_sync(0xFFFFFFFFu, inc[k], off);
+      if ((inside >> lane) & 1u) inc[k] += v;
+    }
+  }
+  return (first >> lane) & 1u;
+}
+
 // Cells [base, base + 32) of one mesh, one per lane of the calling warp
-// (cells past n_cells are masked): compute, optionally aggregate by target
-// point, add with atomics.
+// (cells past n_cells are masked): compute, optionally sum the runs of lanes
+// with one target point, add with atomics.
 template <class L, bool SOA, bool AGG>
 __device__ __forceinline__ void atomic_warp(const LoopData &d, uint32_t base) {
   using out_t = typename L::out_t;
@@ -250,24 +274,7 @@ __device__ __forceinline__ void atomic_warp(const LoopData &d, uint32_t base) {
   for (int s = 0; s < D; ++s) {
     const uint32_t key = valid ? rows.p[0][s] : kNoPoint;
     bool leader = valid;
-    if constexpr (AGG) {
-      const unsigned peers = __match_any_sync(0xFFFFFFFFu, key);
-      const unsigned lt = (1u << lane) - 1u;
-      const int rank = __popc(peers & lt);
-      const int cnt = __popc(peers);
-      const int maxcnt = (int)__reduce_max_sync(0xFFFFFFFFu, (unsigned)cnt);
-      for (int off = 1; off < maxcnt; off <<= 1) {
-        const bool has = rank + off < cnt;
-        const int src = has ? (int)__fns(peers, 0, rank + off + 1) : (int)lane;
-        const bool take = has && (rank % (2 * off)) == 0;
-#pragma unroll
-        for (int k = 0; k < K; ++k) {
-          const out_t v = __shfl_sync(0xFFFFFFFFu, inc[s][k], src);
-          if (take) inc[s][k] += v;
-        }
-      }
-      leader = valid && rank == 0;
-    }
+    if constexpr (AGG) leader = sum_runs<K>(key, inc[s]) && valid;
     if constexpr (!SOA && sizeof(out_t) == 8) {
       __shared__ __align__(16) out_t s_rows[kAtomicWarps][32 * K];
       add_rows_f64<K>(out, s_rows[threadIdx.x >> 5], leader ? key : kNoPoint, inc[s]);

@@ -1,6 +1,7 @@
 """The atomic executor's reductions on the GPU: rows of every width laid out
-across warps of every fill.  Tolerances as for every atomic run: 1e-12 (FP64)
-and 1e-5 (FP32) normwise against the oracle's serial loop."""
+across warps of every fill, and runs of neighbouring cells with one target
+point summed before the reduction.  Tolerances as for every atomic run: 1e-12
+(FP64) and 1e-5 (FP32) normwise against the oracle's serial loop."""
 import numpy as np
 import pytest
 
@@ -43,3 +44,24 @@ def check(md, flags, iters=2):
 @pytest.mark.parametrize("name", list(MESHES))
 def test_rows_of_partly_filled_warps(name, n, layout, flags):
     check(cut(MESHES[name](layout), n), flags)
+
+
+# lengths of the runs of one target point that cells come in
+RUNS = {"all_one": [10 ** 6], "pairs": [2], "threes": [3], "warp": [32], "across_warps": [33],
+        "mixed": [1, 2, 1, 5, 3, 17, 1, 1, 8, 31, 4]}
+
+
+@pytest.mark.parametrize("layout", ["aos", "soa"])
+@pytest.mark.parametrize("runs", list(RUNS))
+@pytest.mark.parametrize("name", ["volna", "getacc"])
+def test_runs_of_one_point(name, runs, layout):
+    md = MESHES[name](layout)
+    g = np.random.default_rng(7)
+    n, dim, points = md.n_cells, md.maps[0].shape[1], md.n_points[0]
+    length = np.resize(np.array(RUNS[runs]), n)
+    run = np.repeat(np.arange(n), length)[:n]
+    # distinct points in a row; neighbouring runs may share a point by chance
+    rows = np.stack([g.permutation(points)[:dim] for _ in range(int(run.max()) + 1)])
+    m = np.ascontiguousarray(rows[run].astype(np.uint32))
+    md.maps = [m] + [m.copy() for _ in md.maps[1:]]
+    check(md, 0)
