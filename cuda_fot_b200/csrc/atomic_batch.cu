@@ -6,6 +6,7 @@
 // ... to keep their symbols apart from the exact ones of batch.cu.
 #define FOT_ADAPTER_ALL 1
 #define FOT_NS_SUFFIX _fma
+#define FOT_CONTRACTED 1  // functors may take a form with fewer operations
 #include "batch.cuh"
 #include "engine.hpp"
 #include "loops.cuh"

@@ -1,7 +1,8 @@
 // miniAero face flux (the per-face user function).
 //
 // Drop-in format of the reference's kernels/mini_aero_func.hpp (same include
-// protocol as res_calc_func.hpp); arithmetic as mini_aero_func.hpp:11-85.
+// protocol as res_calc_func.hpp); arithmetic as mini_aero_func.hpp:11-85, or,
+// where FOT_CONTRACTED is defined, the same flux with fewer operations.
 // Cell records (stride cell_stride): conserved values (5), centre (3),
 // gradients (15), limiters (5); face record (stride face_stride): centre,
 // normal, tangent, binormal.  flux receives the inviscid minus the viscous
@@ -28,6 +29,16 @@ USER_FUNCTION_SIGNATURE(double flux[5], const double *RESTRICT cell_values_left,
                         const double *RESTRICT face_tangent,
                         const double *RESTRICT face_binormal,
                         MY_SIZE cell_stride, MY_SIZE face_stride) {
+#ifdef FOT_CONTRACTED
+  // the atomic executor's form (mini_aero_utils.hpp)
+  double Pl[5], Pr[5];
+  ma_gradient_sums sums = {{0.0, 0.0, 0.0}, 0.0, 0.0};
+  ma_side(cell_values_left, cell_coordinates_left, cell_gradients_left, cell_limiters_left,
+          face_coordinates, face_normal, cell_stride, face_stride, Pl, sums);
+  ma_side(cell_values_right, cell_coordinates_right, cell_gradients_right, cell_limiters_right,
+          face_coordinates, face_normal, cell_stride, face_stride, Pr, sums);
+  ma_face_flux(Pl, Pr, sums, flux, face_normal, face_tangent, face_binormal, face_stride);
+#else
   double Ul[5], Ur[5], Pl[5], Pr[5];
 #pragma unroll
   for (int k = 0; k < 5; ++k) {
@@ -69,6 +80,7 @@ USER_FUNCTION_SIGNATURE(double flux[5], const double *RESTRICT cell_values_left,
                    face_stride);
 #pragma unroll
   for (int k = 0; k < 5; ++k) flux[k] -= vf[k];
+#endif
 }
 
 #undef USER_FUNCTION_SIGNATURE

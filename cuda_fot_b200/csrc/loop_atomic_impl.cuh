@@ -10,6 +10,7 @@
 #pragma once
 
 #define FOT_NS_SUFFIX _fma
+#define FOT_CONTRACTED 1  // functors may take a form with fewer operations
 #include "engine.hpp"
 #include "loops.cuh"
 

@@ -1,7 +1,8 @@
 """The atomic executor's reductions on the GPU: rows of every width laid out
-across warps of every fill, and runs of neighbouring cells with one target
-point summed before the reduction.  Tolerances as for every atomic run: 1e-12
-(FP64) and 1e-5 (FP32) normwise against the oracle's serial loop."""
+across warps of every fill, runs of neighbouring cells with one target point
+summed before the reduction, and the contracted miniAero flux over states the
+generator does not reach.  Tolerances as for every atomic run: 1e-12 (FP64)
+and 1e-5 (FP32) normwise against the oracle's serial loop."""
 import numpy as np
 import pytest
 
@@ -65,3 +66,23 @@ def test_runs_of_one_point(name, runs, layout):
     m = np.ascontiguousarray(rows[run].astype(np.uint32))
     md.maps = [m] + [m.copy() for _ in md.maps[1:]]
     check(md, 0)
+
+
+@pytest.mark.parametrize("layout", ["aos", "soa"])
+def test_contracted_face_flux(layout):
+    """Faces of any area and direction, slow to supersonic flow in each
+    direction (every branch of the eigenvalue fix), steep gradients."""
+    md = mg.mini_aero(9, 6, "aos")
+    g = np.random.default_rng(11)
+    rec, face = md.point_data[1], md.cell_data[0]
+    n = len(rec)
+    rho = g.uniform(0.2, 3.0, n)
+    vel = g.uniform(-2.5, 2.5, (n, 3)) * g.choice([0.01, 0.3, 1.0, 4.0], (n, 1))
+    rec[:, 0] = rho
+    rec[:, 1:4] = rho[:, None] * vel
+    rec[:, 4] = rho * (g.uniform(1.5, 4.0, n) + 0.5 * (vel ** 2).sum(1))
+    rec[:, 8:20] = g.uniform(-2e-2, 2e-2, (n, 12))
+    rec[:, 20:23] = g.uniform(-1e-3, 1e-3, (n, 3))  # of T, which is 2e-3 to 6e-3 here
+    frame = np.linalg.qr(g.normal(size=(md.n_cells, 3, 3)))[0] * g.uniform(0.05, 5.0, (md.n_cells, 1, 3))
+    face[3:12] = frame.transpose(2, 1, 0).reshape(9, -1)
+    check(md.to_layout(layout), 1)
