@@ -566,10 +566,7 @@ static int run_plan(fot_problem *p, fot_plan *plan, uint32_t iterations, cudaStr
     return fail(FOT_ERR_STATE, "plan is stale: the problem's point layout changed after the plan was built");
   if (plan->desc.exec == FOT_EXEC_ATOMIC) {
     const bool agg = !(plan->desc.flags & FOT_PLAN_NO_AGGREGATE);
-    const uint32_t need = (p->n_cells + 255) / 256;
-    const uint32_t grid = std::max<uint32_t>(1, std::min<uint32_t>(need, (uint32_t)(plan->per_sm * sms)));
-    for (uint32_t it = 0; it < iterations; ++it) FOT_TRY(ops->run_atomic(d, soa, agg, 256, grid, st));
-    return FOT_OK;
+    return ops->run_atomic(d, soa, agg, (uint32_t)(plan->per_sm * sms), iterations, st);
   }
   if (plan->version != p->version)
     return fail(FOT_ERR_STATE, "plan is stale: the problem was reordered after the plan was built");

@@ -37,9 +37,10 @@ struct SmemLayout {
 constexpr uint32_t kVariantStage = 1u, kVariantPipe = 2u, kVariantSlots3 = 4u, kVariantSplit = 8u;
 
 struct LoopOps {
-  // launch one iteration of the atomic executor
-  int (*run_atomic)(const LoopData &d, bool soa, bool aggregate, uint32_t threads,
-                    uint32_t grid, cudaStream_t st);
+  // launch `iterations` iterations of the atomic executor; resident: CTAs the
+  // GPU holds at once
+  int (*run_atomic)(const LoopData &d, bool soa, bool aggregate, uint32_t resident,
+                    uint32_t iterations, cudaStream_t st);
   // persistent hierarchical launch over P.total_tiles tiles
   int (*run_hier)(const LoopData &d, const HierPlanDev &P, bool soa, uint32_t threads,
                   uint32_t variant, uint32_t grid, size_t smem, cudaStream_t st);

@@ -2,8 +2,7 @@
 //
 // (a) Global atomics (FOT_EXEC_ATOMIC) -- replaces the reference's
 //     global-colouring executor (problem.hpp:90-194, one launch and one
-//     cudaDeviceSynchronize per colour).  One launch per iteration, one thread
-//     per cell, mapping rows read as vectors, read sets gathered straight from
+//     cudaDeviceSynchronize per colour).  One thread per cell, mapping rows read as vectors, read sets gathered straight from
 //     HBM/L2, increments added with native atomics (f64 RED, AOS rows laid end
 //     to end across the warp first; one 16-byte f32x4 RED per row for the FP32
 //     loop).  With warp aggregation, runs of neighbouring lanes whose
@@ -313,21 +312,51 @@ template <class L> __device__ __forceinline__ void prefetch_cell(const LoopData 
   }
 }
 
-// Persistent grid-stride loop over 32-cell chunks, one chunk per warp at a
-// time; with L::kAtomicPrefetch, in the SOA form, each warp first prefetches
-// the chunk it will take next, so that its mapping rows and direct data come
+// The launch of the atomic executor: tiles of 256 cells (32 per warp), taken
+// in phases.  CTA c of a phase's `resident` CTAs takes tiles first + c,
+// first + c + resident, ...: neighbouring CTAs run side by side through the
+// mesh, so that a row one warp reads as a cell's first point is still in L2
+// when another reads it as a second point.  A CTA that lags behind loses
+// that, lags further, and the launch ends with idle SMs; at a phase's end the
+// CTAs fall into step again (the next phase's CTA starts where one finished
+// first), at the price of a CTA start per phase.  One round a CTA was always
+// slower than several (starts), and which loops drift was measured, R rounds a
+// phase against one phase for all: miniAero SOA 128^3 421 us (R = 4) and 585,
+// 120^3 342 and 352, but 96^3 177 and 172 (23 rounds in all: not split);
+// getacc 1024^2 43.4 and 45.1 (AOS), 1500x1600 SOA 88.7 and 101.1; volna 1024^2
+// 39.8 and 40.9 (R = 8); res_calc 2000x1900 SOA 133 and 130, LULESH 96^3 46.2
+// and 46.2 (never split), miniAero AOS 128^3 489 and 447 (never split).
+//
+// The iterations of a call are one launch as well (no iteration reads what
+// another writes), each running through the mesh in the direction opposite to
+// the one before it, so that it starts on what is left in L2: 10 iterations of
+// res_calc 1000^2 SOA (152 MB each) 391 us as launches of their own, 329 us so
+// (after RCM, data not in L2 before the call); an iteration of 10, warm, of
+// LULESH 96^3 45.2 and 38.1 us, volna 1024^2 41.7 and 29.8, getacc 1024^2 45.9
+// and 34.2 (miniAero 128^3, 1.29 GB, gains its launch gaps only).
+struct AtomicGrid {
+  uint32_t tiles;     // of one iteration
+  uint32_t resident;  // CTAs of a phase
+  uint32_t rounds;    // tiles a CTA takes, at most
+  uint32_t ctas;      // of one iteration: phases * resident
+};
+
+// With L::kAtomicPrefetch, in the SOA form, each warp first prefetches the
+// cells it will take next, so that their mapping rows and direct data come
 // from L2 then.
 template <class L, bool SOA, bool AGG>
-__global__ void __launch_bounds__(256, L::kAtomicMinBlocks) k_atomic(LoopData d) {
-  const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const uint32_t n_warps = (gridDim.x * blockDim.x) >> 5;
-  const uint32_t lane = threadIdx.x & 31u;
-  for (uint32_t base = warp * 32u; base < d.n_cells; base += n_warps * 32u) {
+__global__ void __launch_bounds__(256, L::kAtomicMinBlocks) k_atomic(LoopData d, AtomicGrid g) {
+  const uint32_t in_tile = threadIdx.x & ~31u, lane = threadIdx.x & 31u;
+  const uint32_t it = blockIdx.x / g.ctas, b = blockIdx.x - it * g.ctas;
+  const uint32_t phase = b / g.resident;
+  uint32_t t = phase * g.rounds * g.resident + (b - phase * g.resident);
+  for (uint32_t r = 0; r < g.rounds && t < g.tiles; ++r, t += g.resident) {
     if constexpr (L::kAtomicPrefetch && SOA) {
-      const uint32_t next = base + n_warps * 32u + lane;
-      if (next < d.n_cells) prefetch_cell<L>(d, next);
+      const uint32_t n = t + g.resident;
+      const uint32_t next = ((it & 1u) ? g.tiles - 1u - n : n) * 256u + in_tile + lane;
+      if (r + 1 < g.rounds && n < g.tiles && next < d.n_cells) prefetch_cell<L>(d, next);
     }
-    atomic_warp<L, SOA, AGG>(d, base);
+    atomic_warp<L, SOA, AGG>(d, ((it & 1u) ? g.tiles - 1u - t : t) * 256u + in_tile);
   }
 }
 

@@ -9,6 +9,8 @@
 // (loop_*.cu, -fmad=false) where a run is bit-identical to its CPU replay.
 #pragma once
 
+#include <algorithm>
+
 #define FOT_NS_SUFFIX _fma
 #define FOT_CONTRACTED 1  // functors may take a form with fewer operations
 #include "engine.hpp"
@@ -19,10 +21,26 @@ namespace {
 
 using LA = FOT_LNS(FOT_ADAPTER_NS)::Loop;
 
+// `iterations` iterations in one launch (more only where the grid would grow
+// past 2^30 CTAs).
 template <bool SOA, bool AGG>
-int launch_atomic(const LoopData &d, uint32_t grid, cudaStream_t st) {
-  k_atomic<LA, SOA, AGG><<<grid, 256, 0, st>>>(d);
-  FOT_CUDA(cudaGetLastError());
+int launch_atomic(const LoopData &d, uint32_t resident, uint32_t iterations, cudaStream_t st) {
+  AtomicGrid g;
+  g.tiles = (d.n_cells + 255u) / 256u;
+  g.resident = std::max(1u, std::min(g.tiles, resident));
+  const uint32_t all = (g.tiles + g.resident - 1) / g.resident;
+  const uint32_t phases = LA::kAtomicSplitAbove[SOA] && all > LA::kAtomicSplitAbove[SOA]
+                              ? (all + LA::kAtomicRounds - 1) / LA::kAtomicRounds
+                              : 1;
+  g.rounds = (all + phases - 1) / phases;
+  g.ctas = phases * g.resident;
+  const uint32_t most = std::max(1u, (1u << 30) / g.ctas);
+  while (iterations) {
+    const uint32_t now = std::min(iterations, most);
+    k_atomic<LA, SOA, AGG><<<g.ctas * now, 256, 0, st>>>(d, g);
+    FOT_CUDA(cudaGetLastError());
+    iterations -= now;
+  }
   return FOT_OK;
 }
 
@@ -32,11 +50,12 @@ template <bool SOA, bool AGG> const void *atomic_kernel() {
 
 } // namespace
 
-int FOT_CAT(atomic_run_, FOT_ADAPTER_NS)(const LoopData &d, bool soa, bool agg, uint32_t threads,
-                                         uint32_t grid, cudaStream_t st) {
-  if (threads != 256) return fail(FOT_ERR_ARG, "atomic executor runs 256 threads per CTA");
-  if (soa) return agg ? launch_atomic<true, true>(d, grid, st) : launch_atomic<true, false>(d, grid, st);
-  return agg ? launch_atomic<false, true>(d, grid, st) : launch_atomic<false, false>(d, grid, st);
+int FOT_CAT(atomic_run_, FOT_ADAPTER_NS)(const LoopData &d, bool soa, bool agg, uint32_t resident,
+                                         uint32_t iterations, cudaStream_t st) {
+  if (soa) return agg ? launch_atomic<true, true>(d, resident, iterations, st)
+                      : launch_atomic<true, false>(d, resident, iterations, st);
+  return agg ? launch_atomic<false, true>(d, resident, iterations, st)
+             : launch_atomic<false, false>(d, resident, iterations, st);
 }
 
 int FOT_CAT(atomic_occupancy_, FOT_ADAPTER_NS)(bool soa, bool agg, int *per_sm) {

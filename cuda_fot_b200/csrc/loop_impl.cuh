@@ -11,8 +11,8 @@
 namespace fot {
 
 // the atomic executor of this loop (atomic_*.cu, loop_atomic_impl.cuh)
-int FOT_CAT(atomic_run_, FOT_ADAPTER_NS)(const LoopData &d, bool soa, bool agg, uint32_t threads,
-                                         uint32_t grid, cudaStream_t st);
+int FOT_CAT(atomic_run_, FOT_ADAPTER_NS)(const LoopData &d, bool soa, bool agg, uint32_t resident,
+                                         uint32_t iterations, cudaStream_t st);
 int FOT_CAT(atomic_occupancy_, FOT_ADAPTER_NS)(bool soa, bool agg, int *per_sm);
 
 namespace FOT_ADAPTER_NS {

@@ -54,12 +54,16 @@
 #define FOT_CAT(a, b) FOT_CAT2(a, b)
 #define FOT_LNS(name) FOT_CAT(name, FOT_NS_SUFFIX)
 // Resident CTAs per SM of the atomic executor, per loop (its register cap is
-// 65536 / (256 * this)); measured choices, overridable at build time.
+// 65536 / (256 * this)); measured choices, overridable at build time.  After
+// RCM, AOS / SOA: res_calc 1000^2 5 CTAs 43.0 / 39.4 us, 4: 45.3 / 40.9, 6: 47.5 /
+// 45.5 (aggregated 43.4 / 36.4, 47.6 / 41.3, 47.6 / 36.2); mini_aero 96^3 3 CTAs (80
+// registers) 195 / 172 us, 2: 200 / 182 (4 CTAs spill too much: 321 / 285 with a
+// larger functor).
 #ifndef FOT_ATOMIC_MINB_RES_CALC
-#define FOT_ATOMIC_MINB_RES_CALC 4
+#define FOT_ATOMIC_MINB_RES_CALC 5
 #endif
 #ifndef FOT_ATOMIC_MINB_MINI_AERO
-#define FOT_ATOMIC_MINB_MINI_AERO 2
+#define FOT_ATOMIC_MINB_MINI_AERO 3
 #endif
 #ifndef FOT_ATOMIC_MINB_LULESH
 #define FOT_ATOMIC_MINB_LULESH 2
@@ -69,6 +73,29 @@
 #endif
 #ifndef FOT_ATOMIC_MINB_GETACC
 #define FOT_ATOMIC_MINB_GETACC 2
+#endif
+// Phases of the atomic executor's launch (AtomicGrid): split when a CTA would
+// take more than ABOVE tiles (AOS, SOA; 0: never), into phases of ROUNDS tiles
+// a CTA; the measurements are at AtomicGrid.
+#ifndef FOT_ATOMIC_ABOVE_RES_CALC
+#define FOT_ATOMIC_ABOVE_RES_CALC 0, 0
+#define FOT_ATOMIC_ROUNDS_RES_CALC 1
+#endif
+#ifndef FOT_ATOMIC_ABOVE_MINI_AERO
+#define FOT_ATOMIC_ABOVE_MINI_AERO 0, 24
+#define FOT_ATOMIC_ROUNDS_MINI_AERO 4
+#endif
+#ifndef FOT_ATOMIC_ABOVE_LULESH
+#define FOT_ATOMIC_ABOVE_LULESH 0, 0
+#define FOT_ATOMIC_ROUNDS_LULESH 1
+#endif
+#ifndef FOT_ATOMIC_ABOVE_VOLNA
+#define FOT_ATOMIC_ABOVE_VOLNA 8, 8
+#define FOT_ATOMIC_ROUNDS_VOLNA 8
+#endif
+#ifndef FOT_ATOMIC_ABOVE_GETACC
+#define FOT_ATOMIC_ABOVE_GETACC 4, 4
+#define FOT_ATOMIC_ROUNDS_GETACC 4
 #endif
 // Whether the atomic executor (SOA form) prefetches the next chunk's mapping
 // rows and direct data into L2 while it computes the current one (per loop;
@@ -120,6 +147,9 @@ struct Loop {
   static constexpr int kAtomicMinBlocks = FOT_ATOMIC_MINB_RES_CALC;
   // the atomic executor prefetches the next chunk into L2
   static constexpr bool kAtomicPrefetch = FOT_ATOMIC_PREFETCH_RES_CALC;
+  // phases of its launch: split above so many tiles a CTA (AOS, SOA), this many a phase
+  static constexpr uint32_t kAtomicSplitAbove[2] = {FOT_ATOMIC_ABOVE_RES_CALC};
+  static constexpr uint32_t kAtomicRounds = FOT_ATOMIC_ROUNDS_RES_CALC;
   // read set r: x (set 1, class 1, dim 2), q (set 2, class 0, dim 4), adt (set 3, class 0, dim 1)
   __host__ __device__ static constexpr int read_set(int r) { return r + 1; }
   __host__ __device__ static constexpr int read_class(int r) { return r == 0 ? 1 : 0; }
@@ -164,6 +194,9 @@ struct Loop {
   static constexpr int kAtomicMinBlocks = FOT_ATOMIC_MINB_MINI_AERO;
   // the atomic executor prefetches the next chunk into L2
   static constexpr bool kAtomicPrefetch = FOT_ATOMIC_PREFETCH_MINI_AERO;
+  // phases of its launch: split above so many tiles a CTA (AOS, SOA), this many a phase
+  static constexpr uint32_t kAtomicSplitAbove[2] = {FOT_ATOMIC_ABOVE_MINI_AERO};
+  static constexpr uint32_t kAtomicRounds = FOT_ATOMIC_ROUNDS_MINI_AERO;
   __host__ __device__ static constexpr int read_set(int) { return 1; }
   __host__ __device__ static constexpr int read_class(int) { return 0; }
   __host__ __device__ static constexpr int read_dim(int) { return 28; }
@@ -218,6 +251,9 @@ struct Loop {
   static constexpr int kAtomicMinBlocks = FOT_ATOMIC_MINB_LULESH;
   // the atomic executor prefetches the next chunk into L2
   static constexpr bool kAtomicPrefetch = FOT_ATOMIC_PREFETCH_LULESH;
+  // phases of its launch: split above so many tiles a CTA (AOS, SOA), this many a phase
+  static constexpr uint32_t kAtomicSplitAbove[2] = {FOT_ATOMIC_ABOVE_LULESH};
+  static constexpr uint32_t kAtomicRounds = FOT_ATOMIC_ROUNDS_LULESH;
   __host__ __device__ static constexpr int read_set(int) { return 1; }
   __host__ __device__ static constexpr int read_class(int) { return 0; }
   __host__ __device__ static constexpr int read_dim(int) { return 3; }
@@ -270,6 +306,9 @@ struct Loop {
   static constexpr int kAtomicMinBlocks = FOT_ATOMIC_MINB_VOLNA;
   // the atomic executor prefetches the next chunk into L2
   static constexpr bool kAtomicPrefetch = FOT_ATOMIC_PREFETCH_VOLNA;
+  // phases of its launch: split above so many tiles a CTA (AOS, SOA), this many a phase
+  static constexpr uint32_t kAtomicSplitAbove[2] = {FOT_ATOMIC_ABOVE_VOLNA};
+  static constexpr uint32_t kAtomicRounds = FOT_ATOMIC_ROUNDS_VOLNA;
   __host__ __device__ static constexpr int read_set(int) { return 1; }
   __host__ __device__ static constexpr int read_class(int) { return 0; }
   __host__ __device__ static constexpr int read_dim(int) { return 1; }
@@ -316,6 +355,9 @@ struct Loop {
   static constexpr int kAtomicMinBlocks = FOT_ATOMIC_MINB_GETACC;
   // the atomic executor prefetches the next chunk into L2
   static constexpr bool kAtomicPrefetch = FOT_ATOMIC_PREFETCH_GETACC;
+  // phases of its launch: split above so many tiles a CTA (AOS, SOA), this many a phase
+  static constexpr uint32_t kAtomicSplitAbove[2] = {FOT_ATOMIC_ABOVE_GETACC};
+  static constexpr uint32_t kAtomicRounds = FOT_ATOMIC_ROUNDS_GETACC;
   __host__ __device__ static constexpr int read_set(int) { return 0; }
   __host__ __device__ static constexpr int read_class(int) { return 0; }
   __host__ __device__ static constexpr int read_dim(int) { return 1; }

@@ -86,3 +86,29 @@ def test_contracted_face_flux(layout):
     frame = np.linalg.qr(g.normal(size=(md.n_cells, 3, 3)))[0] * g.uniform(0.05, 5.0, (md.n_cells, 1, 3))
     face[3:12] = frame.transpose(2, 1, 0).reshape(9, -1)
     check(md.to_layout(layout), 1)
+
+
+# meshes around the sizes at which the launch is split into phases: fewer
+# tiles than the GPU holds CTAs, a few rounds, and more rounds than one phase
+SIZES = {"getacc_small": lambda lay: mg.getacc(33, 21, 5, lay), "getacc_phases": lambda lay: mg.getacc(1100, 905, 5, lay),
+         "volna_phases": lambda lay: mg.volna(1003, 997, 5, lay), "res_calc": lambda lay: mg.res_calc(301, 299, 5, lay),
+         "mini_aero_phases": lambda lay: mg.mini_aero(103, 5, lay, permute=False),
+         "lulesh": lambda lay: mg.lulesh(31, 5, lay)}
+
+
+@pytest.mark.parametrize("iters", [1, 2, 5])
+@pytest.mark.parametrize("layout", ["aos", "soa"])
+@pytest.mark.parametrize("name", list(SIZES))
+def test_iterations_of_one_launch(name, layout, iters):
+    """Every cell once per iteration, in either direction through the mesh."""
+    md = SIZES[name](layout)
+    p = F().Problem.from_mesh(md)
+    plan = p.plan(F().EXEC_ATOMIC, 256, F().PLAN_NO_AGGREGATE)
+    plan.run(iters)
+    p.sync()
+    # rel_err is normwise, so one serial iteration scaled up serves as the
+    # oracle of several: the loops never read what they increment (FP64: the
+    # scaling rounds once; FP32 starts from a state of its own)
+    base, one = md.point_data[0].astype(np.float64), O.serial(md, 1)[0][0].astype(np.float64)
+    want = base + iters * (one - base)
+    assert rel_err(p.point_weights(0), want) <= (1e-5 if md.loop == mg.VOLNA else 1e-12)
