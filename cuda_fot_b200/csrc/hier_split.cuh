@@ -61,8 +61,59 @@ __device__ __forceinline__ void griddep_wait() {
   asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
+// A tile's write-back data in the direct form (built by plan.cu): the written
+// points, their slots (0xFFFFFFFF: private), and per point its contributions
+// pc_idx[pc_off[j], pc_off[j + 1]) = slot * threads + cell, in thread-colour
+// order.
+struct DirectRecord {
+  const uint32_t *pts, *wslot;
+  const uint16_t *pc_off, *pc_idx;
+  __host__ __device__ DirectRecord(const unsigned char *r, uint32_t n0)
+      : pts(reinterpret_cast<const uint32_t *>(r)), wslot(pts + n0),
+        pc_off(reinterpret_cast<const uint16_t *>(wslot + n0)), pc_idx(pc_off + n0 + 1) {}
+  // bytes for n0 written points and E contributions, a multiple of 16
+  __host__ __device__ static uint32_t bytes(uint32_t n0, uint32_t E) {
+    return (8u * n0 + 2u * (n0 + 1 + E) + 15u) & ~15u;
+  }
+};
+
+// Row r of K values (side by side) of L2-resident data, in 16-byte loads where
+// rows are a multiple of 16 bytes.
+template <int K, class T> __device__ __forceinline__ void load_row_cg(const T *base, size_t r, T (&v)[K]) {
+  if constexpr (sizeof(T) == 4 && K == 4) {
+    const float4 w = __ldcg(reinterpret_cast<const float4 *>(base) + r);
+    v[0] = w.x;
+    v[1] = w.y;
+    v[2] = w.z;
+    v[3] = w.w;
+  } else if constexpr (sizeof(T) == 8 && K % 2 == 0) {
+#pragma unroll
+    for (int k = 0; k < K; k += 2) {
+      const double2 w = __ldcg(reinterpret_cast<const double2 *>(base + r * K + k));
+      v[k] = w.x;
+      v[k + 1] = w.y;
+    }
+  } else {
+#pragma unroll
+    for (int k = 0; k < K; ++k) v[k] = __ldcg(base + r * K + k);
+  }
+}
+template <int K, class T> __device__ __forceinline__ void store_row_cg(T *base, size_t r, const T (&v)[K]) {
+  if constexpr (sizeof(T) == 4 && K == 4) {
+    __stcg(reinterpret_cast<float4 *>(base) + r, make_float4(v[0], v[1], v[2], v[3]));
+  } else if constexpr (sizeof(T) == 8 && K % 2 == 0) {
+#pragma unroll
+    for (int k = 0; k < K; k += 2)
+      __stcg(reinterpret_cast<double2 *>(base + r * K + k), make_double2(v[k], v[k + 1]));
+  } else {
+#pragma unroll
+    for (int k = 0; k < K; ++k) __stcg(base + r * K + k, v[k]);
+  }
+}
+
 // Shared points [g0, g1) of the previous launch's buffer: out[p] plus the
-// blocks' sums in plan order (thread t of nt).
+// blocks' sums in plan order (thread t of nt, a point a thread: its K sums
+// are independent chains).
 template <class L, bool SOA>
 __device__ __forceinline__ void combine_shared(const LoopData &d, const HierPlanDev &P, uint32_t g0,
                                                uint32_t g1, uint32_t t, uint32_t nt) {
@@ -71,15 +122,25 @@ __device__ __forceinline__ void combine_shared(const LoopData &d, const HierPlan
   const out_t *part = static_cast<const out_t *>(P.partial) + (size_t)(P.put_buf ^ 1u) * P.n_slots * K;
   out_t *out = static_cast<out_t *>(d.out);
   for (uint32_t g = g0 + t; g < g1; g += nt) {
-    const uint32_t p = P.comb_point[g], e0 = P.comb_base[g], e1 = P.comb_base[g + 1];
-    out_t o[K];
+    const uint32_t p = __ldg(P.comb_point + g), e0 = __ldg(P.comb_base + g), e1 = __ldg(P.comb_base + g + 1);
+    out_t o[K], v[K];
+    if constexpr (SOA) {
 #pragma unroll
-    for (int k = 0; k < K; ++k) o[k] = __ldcg(out + out_index(SOA, d.n_points[0], p, K, k));
-    for (uint32_t e = e0; e < e1; ++e)
+      for (int k = 0; k < K; ++k) o[k] = __ldcg(out + out_index(true, d.n_points[0], p, K, k));
+    } else {
+      load_row_cg<K>(out, p, o);
+    }
+    for (uint32_t e = e0; e < e1; ++e) {
+      load_row_cg<K>(part, e, v);
 #pragma unroll
-      for (int k = 0; k < K; ++k) o[k] += __ldcg(part + (size_t)e * K + k);
+      for (int k = 0; k < K; ++k) o[k] += v[k];
+    }
+    if constexpr (SOA) {
 #pragma unroll
-    for (int k = 0; k < K; ++k) __stcg(out + out_index(SOA, d.n_points[0], p, K, k), o[k]);
+      for (int k = 0; k < K; ++k) __stcg(out + out_index(true, d.n_points[0], p, K, k), o[k]);
+    } else {
+      store_row_cg<K>(out, p, o);
+    }
   }
 }
 
@@ -89,45 +150,111 @@ __device__ __forceinline__ void comb_chunk(uint32_t n, uint32_t c, uint32_t part
   g1 = (uint32_t)((uint64_t)n * (c + 1) / parts);
 }
 
-// Written point j of a tile (threads j = t, t + T, ...): sum its contributions
-// in thread-colour order from the increments in shared memory, then add it
-// (private) or store it into its slot of this launch's buffer (shared).
+// How a tile's written points are shared out over its threads.
+// Rows of doubles in AOS data: one (point, component) per thread, so that the
+// K lanes of a point write whole 32-byte sectors (a reduction per sector
+// instead of one per element, see add_rows_f64).  Otherwise one point per
+// thread with its K sums in registers: neighbouring lanes then write
+// neighbouring addresses of each component (SOA), or each a 16-byte row (FP32
+// AOS), and a point's contribution list is walked once.  Direct form, parts of
+// 256, by element and by point: res_calc 1000^2 AOS 63 and 77 us, getacc 1024^2
+// AOS 55 and 77; by point in SOA: res_calc 51 us, 63 by element.
+template <class L, bool SOA> constexpr bool by_element() {
+  return !SOA && sizeof(typename L::out_t) == 8;
+}
+template <class L, bool SOA> constexpr bool by_row4() {
+  return !SOA && sizeof(typename L::out_t) == 4 && L::kOut == 4;
+}
+
+// The increments of a tile in shared memory: entry ie = slot * T + cell holds
+// K values, side by side for AOS point data (a point's lanes, or its one
+// 16-byte load, read one row), component by component for SOA.
 template <class L, bool SOA, int T>
-__device__ __forceinline__ void split_writeback(const LoopData &d, const HierPlanDev &P,
-                                                const RecView<L> &m, const typename L::out_t *inc,
-                                                uint32_t t) {
+__device__ __forceinline__ uint32_t inc_index(uint32_t ie, uint32_t k) {
+  return SOA ? k * (L::kDim * T) + ie : ie * L::kOut + k;
+}
+
+template <class L, bool SOA, int T>
+__device__ __forceinline__ void put_increments(typename L::out_t *inc,
+                                               const typename L::out_t (&v)[L::kDim][L::kOut], uint32_t t) {
+  constexpr int K = L::kOut;
+#pragma unroll
+  for (int q = 0; q < L::kDim; ++q) {
+    if constexpr (by_element<L, SOA>() && K % 2 == 0) {
+#pragma unroll
+      for (int k = 0; k < K; k += 2)
+        *reinterpret_cast<double2 *>(inc + (q * T + t) * K + k) = make_double2(v[q][k], v[q][k + 1]);
+    } else if constexpr (by_row4<L, SOA>()) {
+      *reinterpret_cast<float4 *>(inc + (q * T + t) * 4) = make_float4(v[q][0], v[q][1], v[q][2], v[q][3]);
+    } else {
+#pragma unroll
+      for (int k = 0; k < K; ++k) inc[inc_index<L, SOA, T>(q * T + t, k)] = v[q][k];
+    }
+  }
+}
+
+// All n0 written points of a tile (thread t of T): sum a point's
+// contributions in thread-colour order from the increments in shared memory,
+// then add the sum (private point: this block alone writes it in this
+// iteration) or store it into its slot of this launch's buffer (shared).
+template <class L, bool SOA, int T>
+__device__ __forceinline__ void split_writeback(const LoopData &d, const HierPlanDev &P, uint32_t n0,
+                                                const uint32_t *pts, const uint32_t *wslot,
+                                                const uint16_t *pc_off, const uint16_t *pc_idx,
+                                                const typename L::out_t *inc, uint32_t t) {
   using out_t = typename L::out_t;
-  constexpr int D = L::kDim, K = L::kOut;
+  constexpr int K = L::kOut;
   out_t *out = static_cast<out_t *>(d.out);
   out_t *put = static_cast<out_t *>(P.partial) + (size_t)P.put_buf * P.n_slots * K;
-  const uint32_t *wslot = m.dep;  // split plans: the record's slot list
-  for (uint32_t j = t; j < m.n0; j += T) {
+  if constexpr (by_element<L, SOA>()) {
+    for (uint32_t i = t; i < n0 * (uint32_t)K; i += T) {
+      const uint32_t j = i / K, k = i % K;
+      out_t acc = out_t(0);
+      const uint32_t e1 = pc_off[j + 1];
+      for (uint32_t e = pc_off[j]; e < e1; ++e) acc += inc[inc_index<L, SOA, T>(pc_idx[e], k)];
+      const uint32_t ws = wslot[j];
+      if (ws == 0xFFFFFFFFu) atomicAdd(out + (size_t)pts[j] * K + k, acc);
+      else __stcg(put + (size_t)ws * K + k, acc);
+    }
+    return;
+  }
+  for (uint32_t j = t; j < n0; j += T) {
     out_t acc[K];
 #pragma unroll
     for (int k = 0; k < K; ++k) acc[k] = out_t(0);
-    const uint32_t e0 = m.pc_off[j], e1 = m.pc_off[j + 1];
-    for (uint32_t e = e0; e < e1; ++e) {
-      const uint32_t ie = m.pc_idx[e];
-#pragma unroll
-      for (int k = 0; k < K; ++k) acc[k] += inc[k * D * T + ie];
-    }
-    const uint32_t p = m.pts0[j];
-    const uint32_t ws = wslot[j];
-    if (ws == 0xFFFFFFFFu) {
-      // private point: this block alone writes it in this iteration
-      if constexpr (sizeof(out_t) == 8) {
-#pragma unroll
-        for (int k = 0; k < K; ++k) atomicAdd(out + out_index(SOA, d.n_points[0], p, K, k), acc[k]);
+    const uint32_t e1 = pc_off[j + 1];
+    for (uint32_t e = pc_off[j]; e < e1; ++e) {
+      const uint32_t ie = pc_idx[e];
+      if constexpr (by_row4<L, SOA>()) {
+        const float4 v = *reinterpret_cast<const float4 *>(inc + ie * 4);
+        acc[0] += v.x;
+        acc[1] += v.y;
+        acc[2] += v.z;
+        acc[3] += v.w;
       } else {
 #pragma unroll
-        for (int k = 0; k < K; ++k) {
-          out_t *o = out + out_index(SOA, d.n_points[0], p, K, k);
-          __stcg(o, __ldcg(o) + acc[k]);
-        }
+        for (int k = 0; k < K; ++k) acc[k] += inc[inc_index<L, SOA, T>(ie, k)];
       }
+    }
+    const uint32_t ws = wslot[j];
+    if (ws != 0xFFFFFFFFu) {
+      store_row_cg<K>(put, ws, acc);
+      continue;
+    }
+    const uint32_t p = pts[j];
+    if constexpr (by_row4<L, SOA>()) {
+      out_t o[K];
+      load_row_cg<K>(out, p, o);
+#pragma unroll
+      for (int k = 0; k < K; ++k) o[k] += acc[k];
+      store_row_cg<K>(out, p, o);
     } else {
 #pragma unroll
-      for (int k = 0; k < K; ++k) __stcg(put + (size_t)ws * K + k, acc[k]);
+      for (int k = 0; k < K; ++k) {
+        out_t *o = out + out_index(SOA, d.n_points[0], p, K, k);
+        if constexpr (sizeof(out_t) == 8) atomicAdd(o, acc[k]);
+        else __stcg(o, __ldcg(o) + acc[k]);
+      }
     }
   }
 }
@@ -135,14 +262,15 @@ __device__ __forceinline__ void split_writeback(const LoopData &d, const HierPla
 // Direct form: CTAs [0, n_blocks) run one tile each, the comb_ctas after
 // them combine the previous buffer (hardware CTA scheduling keeps several tiles per SM in
 // different phases; a persistent form with one tile in flight per CTA and
-// the next tile's plan data prefetched measured slower).  A tile is the
-// reference's block step with HBM/L2 gathers: one thread per cell gathers its
-// rows through the plan-ordered mapping and computes its increments in
-// registers; the increments go into a zeroed shared-memory sum one thread
-// colour after another (cells of one colour write disjoint points: the
-// replay's order, bit for bit); then each written point's sum goes out (RED
-// for private points, the slot for shared ones).  The tile header (start,
-// cells | colours << 16, written points, their offset) is one 16-byte load.
+// the next tile's plan data prefetched measured slower).  One thread per cell
+// gathers its rows through the plan-ordered mapping straight from HBM/L2 and
+// puts its increments into shared memory; after ONE barrier each written
+// point's contributions are summed in thread-colour order (the replay's
+// order, bit for bit) and go out (RED for private points, the slot for shared
+// ones).  What the write-back needs -- points, slots, contribution lists -- is
+// one record per tile (DirectRecord), bulk-copied while the cells compute; the
+// tile header (start, cells | colours << 16, written points, record offset)
+// is one 16-byte load.
 template <class L, int T> constexpr int dsplit_min_blocks() {
   return (65536 / (T * L::kDirectRegCap)) > 0 ? 65536 / (T * L::kDirectRegCap) : 1;
 }
@@ -152,8 +280,9 @@ __global__ void __launch_bounds__(T, dsplit_min_blocks<L, T>()) k_hier_dsplit(Lo
   using out_t = typename L::out_t;
   using read_t = typename L::read_t;
   constexpr int D = L::kDim, K = L::kOut;
-  extern __shared__ __align__(16) unsigned char smem[];
-  out_t *const acc = reinterpret_cast<out_t *>(smem);
+  extern __shared__ __align__(128) unsigned char smem[];
+  __shared__ __align__(8) uint64_t s_full;
+  out_t *const inc = reinterpret_cast<out_t *>(smem + P.inc_off);
   const uint32_t tid = threadIdx.x;
   griddep_launch_dependents();
   const uint32_t n_tiles = P.tiles_on ? P.n_blocks : 0u;
@@ -169,69 +298,38 @@ __global__ void __launch_bounds__(T, dsplit_min_blocks<L, T>()) k_hier_dsplit(Lo
     return;
   }
   const uint4 h = __ldg(P.tile_hdr + blockIdx.x);
-  const uint32_t start = h.x, ncell = h.y & 0xFFFFu, ntcol = h.y >> 16, n0 = h.z, poff = h.w;
-  for (uint32_t e = tid; e < n0 * K; e += T) acc[e] = out_t(0);
-  // this thread's first written point (issued early; used after the sums)
-  uint32_t p_first = 0, ws_first = 0;
-  if (tid < n0) {
-    p_first = __ldg(P.pts[0] + poff + tid);
-    ws_first = __ldg(P.wslot + poff + tid);
+  const uint32_t start = h.x, ncell = h.y & 0xFFFFu, n0 = h.z;
+  if (tid == 0) {
+    const uint32_t bytes = DirectRecord::bytes(n0, D * ncell);
+    mbar_init(&s_full, 1);
+    mbar_fence_init();
+    mbar_expect_tx(&s_full, bytes);
+    bulk_copy_g2s(smem, P.rec + (size_t)h.w * 16, bytes, &s_full);
   }
   if constexpr (L::kWritesCell) griddep_wait();  // the previous iteration may still write cell data
-  const bool active = tid < ncell;
-  const uint32_t pos = start + tid;
-  uint32_t my_col = 0xFFFFFFFFu;
-  uint16_t l0[D];
-  out_t v[D][K];
-  if (active) {
+  if (tid < ncell) {
+    const uint32_t pos = start + tid;
     GlobalRows<L, SOA> rows;
     load_row<D>(d.map[0], pos, rows.p[0]);
     if constexpr (L::kHasClass1) load_row<D>(d.map[1], pos, rows.p[1]);
-#pragma unroll
-    for (int q = 0; q < D; ++q) l0[q] = __ldg(P.lidx[0] + (size_t)q * d.n_cells + pos);
-    my_col = __ldg(P.tcol + pos);
     static_for_read<L>([&](auto r) {
       constexpr int R = decltype(r)::value;
       rows.base[R] = static_cast<const read_t *>(d.point[L::read_set(R)]);
       rows.np[R] = d.n_points[L::read_set(R)];
     });
+    out_t v[D][K];
     Direct dir{d.cell, pos, d.n_cells};
     L::cell(rows, dir, v);
+    put_increments<L, SOA, T>(inc, v, tid);
   }
-  __syncthreads();  // the sums are zeroed
-  for (uint32_t col = 0; col < ntcol; ++col) {
-    if (my_col == col) {
-#pragma unroll
-      for (int q = 0; q < D; ++q)
-#pragma unroll
-        for (int k = 0; k < K; ++k) acc[(uint32_t)l0[q] * K + k] += v[q][k];
-    }
-    __syncthreads();
+  __syncthreads();
+  if (!mbar_wait(&s_full, 0)) {
+    if (tid == 0) atomicOr(&P.ctl->error, kErrWaitLimit);
+    return;
   }
   if constexpr (!L::kWritesCell) griddep_wait();  // the previous iteration's writes are visible
-  out_t *out = static_cast<out_t *>(d.out);
-  out_t *put = static_cast<out_t *>(P.partial) + (size_t)P.put_buf * P.n_slots * K;
-  for (uint32_t j = tid; j < n0; j += T) {
-    const uint32_t p = j == tid ? p_first : __ldg(P.pts[0] + poff + j);
-    const uint32_t ws = j == tid ? ws_first : __ldg(P.wslot + poff + j);
-    const out_t *a = acc + (size_t)j * K;
-    if (ws == 0xFFFFFFFFu) {
-      // private point: this block alone writes it in this iteration
-      if constexpr (sizeof(out_t) == 8) {
-#pragma unroll
-        for (int k = 0; k < K; ++k) atomicAdd(out + out_index(SOA, d.n_points[0], p, K, k), a[k]);
-      } else {
-#pragma unroll
-        for (int k = 0; k < K; ++k) {
-          out_t *o = out + out_index(SOA, d.n_points[0], p, K, k);
-          __stcg(o, __ldcg(o) + a[k]);
-        }
-      }
-    } else {
-#pragma unroll
-      for (int k = 0; k < K; ++k) __stcg(put + (size_t)ws * K + k, a[k]);
-    }
-  }
+  const DirectRecord m(smem, n0);
+  split_writeback<L, SOA, T>(d, P, n0, m.pts, m.wslot, m.pc_off, m.pc_idx, inc, tid);
 }
 
 template <class L, bool SOA, int T, uint32_t kRecSlots>
@@ -373,10 +471,7 @@ __global__ void __launch_bounds__(T + 64) __maxnreg__(L::kRegCap)
         out_t v[D][K];
         Direct dir{d.cell, m.start + tid, d.n_cells};
         L::cell(rv, dir, v);
-#pragma unroll
-        for (int q = 0; q < D; ++q)
-#pragma unroll
-          for (int k = 0; k < K; ++k) inc[(k * D + q) * T + tid] = v[q][k];
+        put_increments<L, SOA, T>(inc, v, tid);
       }
       named_bar_sync<T>();
       if (tid == 0) mbar_arrive(&s_rows_empty[b]);  // the row slot may be refilled
@@ -394,7 +489,8 @@ __global__ void __launch_bounds__(T + 64) __maxnreg__(L::kRegCap)
           combine_shared<L, SOA>(d, P, g0, g1, tid, T);
         }
       }
-      split_writeback<L, SOA, T>(d, P, m, inc, tid);
+      split_writeback<L, SOA, T>(d, P, m.n0, m.pts0, m.dep /* split plans: the slot list */, m.pc_off,
+                                 m.pc_idx, inc, tid);
       __syncwarp();
       if (lane == 0) mbar_arrive(&s_tile_done[s]);
       // the increments buffer is reused by the next tile

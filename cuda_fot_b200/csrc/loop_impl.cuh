@@ -107,7 +107,7 @@ int run_hier(const LoopData &d, const HierPlanDev &P, bool soa, uint32_t threads
     // whatever precedes it may write the datasets it reads.
     const uint32_t iters = P.n_blocks ? P.total_tiles / P.n_blocks : 0;
     const bool direct = !(variant & kVariantPipe);
-    const uint32_t comb_ctas = P.n_shared ? (P.n_shared + 4 * threads - 1) / (4 * threads) : 0;
+    const uint32_t comb_ctas = (P.n_shared + threads - 1) / threads;  // a point a thread
     const void *flush = soa ? dsplit_kernel<true>(threads) : dsplit_kernel<false>(threads);
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -169,9 +169,10 @@ void smem_layout(uint32_t cap0, uint32_t cap1, uint32_t variant, uint32_t rec_ca
   SmemLayout s;
   size_t off = 0;
   if ((variant & kVariantSplit) && !(variant & kVariantPipe)) {
-    // direct split write-back: the block's sums only
-    s.acc_off = 0;
-    s.total = a16((size_t)cap0 * L::kOut * sizeof(out_t));
+    // direct split write-back: the tile's record and the increments
+    s.rec_slot = rec_cap;
+    s.inc_off = (uint32_t)((rec_cap + 127u) & ~127u);
+    s.total = s.inc_off + (size_t)L::kOut * L::kDim * threads * sizeof(out_t);
     *out = s;
     return;
   }

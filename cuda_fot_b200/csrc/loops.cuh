@@ -97,6 +97,13 @@
 #define FOT_ATOMIC_ABOVE_GETACC 4, 4
 #define FOT_ATOMIC_ROUNDS_GETACC 4
 #endif
+// kDirectRegCap of the adapters below: registers per thread that the direct split
+// write-back kernel is held to; its tiles wait for memory at every step, so
+// that the CTAs an SM holds decide.  Parts of 256, AOS / SOA, by cap: res_calc
+// 1000^2 40: 54.7 / 49.7 us, 48: 59.5 / 50.6, 56: 65.6 / 57.1; volna 1024^2 32: 53.8 / 64.3,
+// 40: 64.7 / 82.1, 24: 65.9 / 82.7 (spills); parts of 128: LULESH 96^3 80: 92.7 /
+// 88.2, 72: 109 / 108 (spills), 96: 95.4 / 89.4; getacc 1024^2 56: 49.6 / 47.3, 48: 59.0 /
+// 53.2, 64: 53.3 / 49.6; miniAero hardly moves between 84 and 128.
 // Whether the atomic executor (SOA form) prefetches the next chunk's mapping
 // rows and direct data into L2 while it computes the current one (per loop;
 // measured choices, overridable at build time: on for mini_aero's 96-byte
@@ -142,7 +149,7 @@ struct Loop {
   static constexpr bool kHasClass1 = true;
   static constexpr int kRegCap = 64; // registers per thread the tile kernels are held to
   // registers per thread of the direct split write-back kernel
-  static constexpr int kDirectRegCap = 48;
+  static constexpr int kDirectRegCap = 40;
   // resident 256-thread CTAs per SM the atomic executor is compiled for
   static constexpr int kAtomicMinBlocks = FOT_ATOMIC_MINB_RES_CALC;
   // the atomic executor prefetches the next chunk into L2
@@ -246,7 +253,7 @@ struct Loop {
   static constexpr bool kHasClass1 = false;
   static constexpr int kRegCap = 96; // registers per thread the tile kernels are held to
   // registers per thread of the direct split write-back kernel
-  static constexpr int kDirectRegCap = kRegCap;
+  static constexpr int kDirectRegCap = 80;
   // resident 256-thread CTAs per SM the atomic executor is compiled for
   static constexpr int kAtomicMinBlocks = FOT_ATOMIC_MINB_LULESH;
   // the atomic executor prefetches the next chunk into L2
@@ -301,7 +308,7 @@ struct Loop {
   static constexpr bool kHasClass1 = false;
   static constexpr int kRegCap = 64; // registers per thread the tile kernels are held to
   // registers per thread of the direct split write-back kernel
-  static constexpr int kDirectRegCap = kRegCap;
+  static constexpr int kDirectRegCap = 32;
   // resident 256-thread CTAs per SM the atomic executor is compiled for
   static constexpr int kAtomicMinBlocks = FOT_ATOMIC_MINB_VOLNA;
   // the atomic executor prefetches the next chunk into L2
@@ -350,7 +357,7 @@ struct Loop {
   static constexpr bool kHasClass1 = false;
   static constexpr int kRegCap = 96; // registers per thread the tile kernels are held to
   // registers per thread of the direct split write-back kernel
-  static constexpr int kDirectRegCap = kRegCap;
+  static constexpr int kDirectRegCap = 56;
   // resident 256-thread CTAs per SM the atomic executor is compiled for
   static constexpr int kAtomicMinBlocks = FOT_ATOMIC_MINB_GETACC;
   // the atomic executor prefetches the next chunk into L2

@@ -387,6 +387,60 @@ __global__ void k_build_records(RecordArgs a) {
   for (uint32_t i = used + threadIdx.x; i < a.rec_off[b + 1] - a.rec_off[b]; i += blockDim.x) r[i] = 0;
 }
 
+// The direct form's records (DirectRecord, hier_split.cuh): the same lists
+// without what only the staged form reads.  Cells of one thread colour write
+// disjoint points, so that, colour by colour, each cell appends its entries to
+// its points' lists: one step per colour instead of a scan of all entries per
+// point.
+struct DirectRecordArgs {
+  const uint4 *hdr;               // per tile, see HierPlanDev::tile_hdr
+  const uint32_t *pts_first;      // per tile: its first written point in pts / wslot
+  const uint32_t *pts, *wslot;
+  const uint16_t *lidx;
+  const uint8_t *tcol;
+  unsigned char *rec;
+  uint32_t n_cells, threads;
+  int D;
+};
+
+__global__ void k_build_direct_records(DirectRecordArgs a) {
+  extern __shared__ uint32_t at[];  // per written point: where its next entry goes
+  const uint4 h = a.hdr[blockIdx.x];
+  const uint32_t start = h.x, ncell = h.y & 0xFFFFu, ntcol = h.y >> 16, n0 = h.z;
+  const uint32_t first = a.pts_first[blockIdx.x], E = a.D * ncell;
+  unsigned char *r = a.rec + (size_t)h.w * 16;
+  uint32_t *pts = reinterpret_cast<uint32_t *>(r), *wslot = pts + n0;
+  uint16_t *pc_off = reinterpret_cast<uint16_t *>(wslot + n0), *pc_idx = pc_off + n0 + 1;
+  for (uint32_t j = threadIdx.x; j <= n0; j += blockDim.x) at[j] = 0;
+  for (uint32_t j = threadIdx.x; j < n0; j += blockDim.x) {
+    pts[j] = a.pts[first + j];
+    wslot[j] = a.wslot[first + j];
+  }
+  __syncthreads();
+  for (uint32_t i = threadIdx.x; i < ncell; i += blockDim.x)
+    for (int q = 0; q < a.D; ++q) atomicAdd(&at[a.lidx[(size_t)q * a.n_cells + start + i]], 1u);
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    uint32_t sum = 0;
+    for (uint32_t j = 0; j <= n0; ++j) {
+      const uint32_t c = at[j];
+      at[j] = sum;
+      pc_off[j] = (uint16_t)sum;
+      sum += c;
+    }
+  }
+  __syncthreads();
+  for (uint32_t col = 0; col < ntcol; ++col) {
+    for (uint32_t i = threadIdx.x; i < ncell; i += blockDim.x)
+      if (a.tcol[start + i] == col)
+        for (int q = 0; q < a.D; ++q)
+          pc_idx[at[a.lidx[(size_t)q * a.n_cells + start + i]]++] = (uint16_t)(q * a.threads + i);
+    __syncthreads();
+  }
+  uint16_t *end = reinterpret_cast<uint16_t *>(r + DirectRecord::bytes(n0, E));
+  for (uint16_t *w = pc_idx + E + threadIdx.x; w < end; w += blockDim.x) *w = 0;
+}
+
 // ---------------------------------------------------------------------------
 // step 5: permute the problem's cells (rows of the mappings, cell datasets)
 // ---------------------------------------------------------------------------
@@ -705,6 +759,7 @@ int build_hier_plan(fot_problem *p, fot_plan *plan) {
   // 4b. tile records
   {
     const bool split = plan->variant & kVariantSplit;
+    const bool direct = split && !(plan->variant & kVariantPipe);
     std::vector<uint32_t> final_of(nfb);
     for (uint32_t b = 0; b < nfb; ++b) final_of[order[b]] = b;
     // conflict neighbours of each block in final order; bit 31: earlier
@@ -718,7 +773,7 @@ int build_hier_plan(fot_problem *p, fot_plan *plan) {
       }
       dep_off[b + 1] = (uint32_t)dep.size();
     }
-    DevBuf d_dep_off, d_dep, d_split;
+    DevBuf d_dep_off, d_dep, d_split, d_first;
     FOT_TRY(upload(d_dep_off, dep_off));
     FOT_TRY(upload(d_dep, dep));
     SplitRecords sr;
@@ -736,57 +791,84 @@ int build_hier_plan(fot_problem *p, fot_plan *plan) {
       FOT_TRY(upload(plan->comb_point, sr.point));
       FOT_TRY(upload(plan->comb_base, sr.base));
       FOT_TRY(upload(plan->launch, final_of));
-      FOT_TRY(upload(plan->wslot, sr.wslot));
       // direct form: one 16-byte header per tile, in launch order
+      std::vector<uint32_t> drec_off(nfb + 1, 0);  // direct records, in units of 16 bytes
+      for (uint32_t b = 0; b < nfb; ++b) {
+        const uint32_t bytes = DirectRecord::bytes(h_off[0][b + 1] - h_off[0][b],
+                                                   D * (block_start[b + 1] - block_start[b]));
+        drec_off[b + 1] = drec_off[b] + bytes / 16;
+        if (direct) plan->rec_cap = std::max(plan->rec_cap, bytes);
+      }
       std::vector<uint32_t> hdr((size_t)4 * nfb);
       for (uint32_t t = 0; t < nfb; ++t) {
         const uint32_t b = final_of[t], fb = order[b];
         hdr[4 * t + 0] = block_start[b];
         hdr[4 * t + 1] = (block_start[b + 1] - block_start[b]) | ((uint32_t)h_ntcol[fb] << 16);
         hdr[4 * t + 2] = h_off[0][b + 1] - h_off[0][b];
-        hdr[4 * t + 3] = h_off[0][b];
+        hdr[4 * t + 3] = drec_off[b];
       }
       FOT_TRY(upload(plan->tile_hdr, hdr));
+      if (direct) {
+        std::vector<uint32_t> first(nfb);
+        for (uint32_t t = 0; t < nfb; ++t) first[t] = h_off[0][final_of[t]];
+        FOT_TRY(upload(d_first, first));
+        FOT_TRY(plan->rec.alloc((size_t)drec_off[nfb] * 16));
+        DirectRecordArgs da{};
+        da.hdr = plan->tile_hdr.as<uint4>();
+        da.pts_first = d_first.as<uint32_t>();
+        da.pts = plan->pts[0].as<uint32_t>();
+        da.wslot = d_split.as<uint32_t>();
+        da.lidx = plan->lidx[0].as<uint16_t>();
+        da.tcol = plan->tcol.as<uint8_t>();
+        da.rec = plan->rec.as<unsigned char>();
+        da.n_cells = n;
+        da.threads = hier_threads(B);
+        da.D = D;
+        k_build_direct_records<<<nfb, 128, (plan->cap[0] + 1) * sizeof(uint32_t)>>>(da);
+        FOT_CUDA(cudaGetLastError());
+      }
       plan->n_slots = sr.n_slots;
       plan->n_shared_points = (uint32_t)sr.point.size();
     }
-    std::vector<uint32_t> rec_off(nfb + 1, 0);
-    uint32_t rec_cap = 0;
-    for (uint32_t b = 0; b < nfb; ++b) {
-      const uint32_t ncell = block_start[b + 1] - block_start[b];
-      const uint32_t n0 = h_off[0][b + 1] - h_off[0][b];
-      const uint32_t n1 = n_class > 1 ? h_off[1][b + 1] - h_off[1][b] : 0;
-      uint32_t padded = record_bytes(ncell, n0, n1, D, n_class, dep_off[b + 1] - dep_off[b]);
-      if (split) padded = (record_dep_offset(ncell, n0, n1, D, n_class) + 4 * n0 + 15) & ~15u;
-      rec_cap = std::max(rec_cap, padded);
-      rec_off[b + 1] = rec_off[b] + padded;
-    }
-    FOT_TRY(upload(plan->rec_off, rec_off));
-    FOT_TRY(plan->rec.alloc(rec_off[nfb]));
-    plan->rec_cap = rec_cap;
     // completed iterations of each block (the dependency flags)
     FOT_TRY(plan->block_done.alloc((size_t)nfb * 4));
     FOT_CUDA(cudaMemset(plan->block_done.ptr, 0, (size_t)nfb * 4));
-    RecordArgs ra{};
-    ra.block_start = plan->block_start.as<uint32_t>();
-    ra.block_wait = plan->block_wait.as<uint32_t>();
-    ra.rec_off = plan->rec_off.as<uint32_t>();
-    ra.threads = hier_threads(B);
-    ra.dep_off = d_dep_off.as<uint32_t>();
-    ra.dep = d_dep.as<uint32_t>();
-    ra.wslot = split ? d_split.as<uint32_t>() : nullptr;
-    ra.ntcol = plan->block_ntcol.as<uint8_t>();
-    ra.rec = plan->rec.as<unsigned char>();
-    ra.n_cells = n;
-    ra.n_class = n_class;
-    ra.D = D;
-    for (int c = 0; c < n_class; ++c) {
-      ra.pts_off[c] = plan->pts_off[c].as<uint32_t>();
-      ra.pts[c] = plan->pts[c].as<uint32_t>();
-      ra.lidx[c] = plan->lidx[c].as<uint16_t>();
+    if (!direct) {
+      std::vector<uint32_t> rec_off(nfb + 1, 0);
+      uint32_t rec_cap = 0;
+      for (uint32_t b = 0; b < nfb; ++b) {
+        const uint32_t ncell = block_start[b + 1] - block_start[b];
+        const uint32_t n0 = h_off[0][b + 1] - h_off[0][b];
+        const uint32_t n1 = n_class > 1 ? h_off[1][b + 1] - h_off[1][b] : 0;
+        uint32_t padded = record_bytes(ncell, n0, n1, D, n_class, dep_off[b + 1] - dep_off[b]);
+        if (split) padded = (record_dep_offset(ncell, n0, n1, D, n_class) + 4 * n0 + 15) & ~15u;
+        rec_cap = std::max(rec_cap, padded);
+        rec_off[b + 1] = rec_off[b] + padded;
+      }
+      FOT_TRY(upload(plan->rec_off, rec_off));
+      FOT_TRY(plan->rec.alloc(rec_off[nfb]));
+      plan->rec_cap = rec_cap;
+      RecordArgs ra{};
+      ra.block_start = plan->block_start.as<uint32_t>();
+      ra.block_wait = plan->block_wait.as<uint32_t>();
+      ra.rec_off = plan->rec_off.as<uint32_t>();
+      ra.threads = hier_threads(B);
+      ra.dep_off = d_dep_off.as<uint32_t>();
+      ra.dep = d_dep.as<uint32_t>();
+      ra.wslot = split ? d_split.as<uint32_t>() : nullptr;
+      ra.ntcol = plan->block_ntcol.as<uint8_t>();
+      ra.rec = plan->rec.as<unsigned char>();
+      ra.n_cells = n;
+      ra.n_class = n_class;
+      ra.D = D;
+      for (int c = 0; c < n_class; ++c) {
+        ra.pts_off[c] = plan->pts_off[c].as<uint32_t>();
+        ra.pts[c] = plan->pts[c].as<uint32_t>();
+        ra.lidx[c] = plan->lidx[c].as<uint16_t>();
+      }
+      k_build_records<<<nfb, 128>>>(ra);
+      FOT_CUDA(cudaGetLastError());
     }
-    k_build_records<<<nfb, 128>>>(ra);
-    FOT_CUDA(cudaGetLastError());
   }
 
   // 5. permute the problem's cells into plan order
