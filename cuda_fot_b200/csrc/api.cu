@@ -163,7 +163,6 @@ fot::HierPlanDev fot_plan::dev(uint32_t iterations) const {
   P.outbuf_off = layout.outbuf_off;
   P.outbuf_bytes = layout.outbuf_bytes;
   P.block_done = block_done.as<unsigned int>();
-  P.launch = launch.as<uint32_t>();
   P.partial = partial.ptr;
   P.comb_point = comb_point.as<uint32_t>();
   P.tile_hdr = tile_hdr.as<uint4>();
@@ -393,17 +392,17 @@ int fot_plan_build(fot_problem *p, const fot_plan_desc *desc, fot_plan **out) {
     const uint32_t agg = (desc->flags & FOT_PLAN_NO_AGGREGATE) ? 0u : 1u;
     rc = ops->occupancy(FOT_EXEC_ATOMIC, p->layout == FOT_SOA, 256, agg, 0, &plan->per_sm);
   } else if (desc->exec == FOT_EXEC_HIER || desc->exec == FOT_EXEC_HIER_LAUNCH) {
-    // Persistent executor (blocks of at most 512 cells): the staged split
-    // write-back kernel by default, the direct split write-back kernel with
-    // FOT_PLAN_DIRECT_READS, the pipelined kernel with per-block completion
-    // flags with FOT_PLAN_BLOCK_FLAGS; FOT_PLAN_SIMPLE_TILES (or larger
-    // blocks) selects the simple persistent kernel, staged or direct.
+    // Persistent executor (blocks of at most 512 cells): the split write-back
+    // kernel by default, the pipelined kernel with per-block completion
+    // flags with FOT_PLAN_BLOCK_FLAGS (unless reads are direct);
+    // FOT_PLAN_SIMPLE_TILES (or larger blocks) selects the simple persistent
+    // kernel, staged or direct.
     const bool direct = desc->flags & FOT_PLAN_DIRECT_READS;
     plan->variant = direct ? 0u : kVariantStage;
     if (desc->exec == FOT_EXEC_HIER && desc->block_size <= 512 &&
         !(desc->flags & FOT_PLAN_SIMPLE_TILES)) {
-      if (direct) plan->variant |= kVariantSplit;
-      else plan->variant |= kVariantPipe | ((desc->flags & FOT_PLAN_BLOCK_FLAGS) ? 0u : kVariantSplit);
+      if (!direct && (desc->flags & FOT_PLAN_BLOCK_FLAGS)) plan->variant |= kVariantPipe;
+      else plan->variant = kVariantSplit;
     }
     rc = build_hier_plan(p, plan);
     if (rc == FOT_OK) {
@@ -429,11 +428,18 @@ int fot_plan_build(fot_problem *p, const fot_plan_desc *desc, fot_plan **out) {
       // the pipelined kernel holds two tiles' rows; when they do not fit,
       // the single-buffer persistent kernel runs the plan instead
       if ((plan->variant & kVariantPipe) && plan->layout.total > 227 * 1024) {
-        plan->variant &= ~(kVariantPipe | kVariantSplit);
+        plan->variant &= ~kVariantPipe;
         ops->smem_layout(plan->cap[0], plan->cap[1], plan->variant, plan->rec_cap,
                          plan->threads, &plan->layout);
       }
       plan->smem = plan->layout.total;
+      // A default plan is also what a batch runs, as staged tiles, one at a
+      // time: blocks whose rows and sums do not fit are refused here.
+      if ((plan->variant & kVariantSplit) && !direct) {
+        SmemLayout staged;
+        ops->smem_layout(plan->cap[0], plan->cap[1], kVariantStage, 0, plan->threads, &staged);
+        plan->smem = std::max(plan->smem, staged.total > 227 * 1024 ? staged.total : 0);
+      }
       if (plan->smem > 227 * 1024)
         rc = fail(FOT_ERR_LIMIT,
                   "a block needs %zu bytes of shared memory (limit 227 KB): use a smaller block "
@@ -446,7 +452,7 @@ int fot_plan_build(fot_problem *p, const fot_plan_desc *desc, fot_plan **out) {
     if (rc == FOT_OK && plan->per_sm == 0 && (plan->variant & kVariantPipe)) {
       // the two-tile layout fits the limit but not beside the kernel's own
       // shared memory: the single-buffer persistent kernel runs the plan
-      plan->variant &= ~(kVariantPipe | kVariantSplit);
+      plan->variant &= ~kVariantPipe;
       ops->smem_layout(plan->cap[0], plan->cap[1], plan->variant, plan->rec_cap, plan->threads,
                        &plan->layout);
       plan->smem = plan->layout.total;
@@ -489,7 +495,7 @@ int fot_plan_build(fot_problem *p, const fot_plan_desc *desc, fot_plan **out) {
   if (desc->exec == FOT_EXEC_HIER_LAUNCH) kname = "per-colour launches";
   else if (desc->exec == FOT_EXEC_HIER)
     kname = (plan->variant & kVariantSplit)
-                ? ((plan->variant & kVariantPipe) ? "split write-back" : "split write-back, direct")
+                ? ((desc->flags & FOT_PLAN_DIRECT_READS) ? "split write-back, direct" : "split write-back")
             : (plan->variant & kVariantPipe) ? "pipelined, block flags"
             : (plan->variant & kVariantStage) ? "simple persistent"
                                                : "simple persistent, direct reads";
@@ -573,13 +579,10 @@ static int run_plan(fot_problem *p, fot_plan *plan, uint32_t iterations, cudaStr
     if ((uint64_t)iterations * plan->n_blocks + (uint64_t)plan->per_sm * sms >= 0xFFFFFFFFull)
       return fail(FOT_ERR_LIMIT, "too many tiles in one launch");
     const HierPlanDev P = plan->dev(iterations);
-    // the split kernels run one iteration per launch over the plan's blocks:
-    // persistent CTAs (staged form) or one CTA per block (direct form)
-    const bool split = plan->variant & kVariantSplit;
-    const uint32_t tiles = split ? plan->n_blocks : P.total_tiles;
-    const uint32_t grid = (split && !(plan->variant & kVariantPipe))
+    // the split kernel runs one iteration per launch, one CTA per block
+    const uint32_t grid = (plan->variant & kVariantSplit)
                               ? plan->n_blocks
-                              : std::min<uint32_t>(tiles, (uint32_t)(plan->per_sm * sms));
+                              : std::min<uint32_t>(P.total_tiles, (uint32_t)(plan->per_sm * sms));
     return ops->run_hier(d, P, soa, plan->threads, plan->variant, grid, plan->smem, st);
   }
   const HierPlanDev P = plan->dev(1);
@@ -623,7 +626,7 @@ int fot_sync(fot_problem *p, void *stream) {
 
 int fot_plan_inject_lost_flag(fot_plan *plan, uint32_t block) {
   if (!plan) return fail(FOT_ERR_ARG, "null plan");
-  if (!(plan->variant & kVariantPipe) || (plan->variant & kVariantSplit) || !plan->block_done.ptr)
+  if (!(plan->variant & kVariantPipe) || !plan->block_done.ptr)
     return fail(FOT_ERR_STATE, "the plan does not run the block-flag hierarchical kernel");
   if (block >= plan->n_blocks) return fail(FOT_ERR_ARG, "block %u out of range (%u blocks)", block, plan->n_blocks);
   FOT_CUDA(cudaDeviceSynchronize());

@@ -24,7 +24,7 @@
 //     with has been written back: every tile of the earlier colours for the
 //     simple kernel (k_hier, hier.cuh), the conflicting blocks' completion
 //     flags for the pipelined warp-specialised kernel (k_hier_pipe,
-//     hier_pipe.cuh).  The split write-back kernel (k_hier_split,
+//     hier_pipe.cuh).  The split write-back kernel (k_hier_dsplit,
 //     hier_split.cuh, the default) makes no tile wait: points written by one
 //     block are added at once, points shared by several blocks through
 //     per-block partial sums that the next launch (or a final combine-only
@@ -76,18 +76,17 @@ struct HierPlanDev {
   uint32_t outbuf_off;         // first prefetched-output-row slot
   uint32_t outbuf_bytes;       // bytes of one output-row slot
   unsigned int *block_done;    // per block: completed iterations (relative to ctl->base)
-  // split write-back kernels
-  const uint32_t *launch;      // tile -> block (formation order)
+  // split write-back kernel
   void *partial;               // 2 x n_slots partial-sum rows (AOS, point dataset 0's type)
   const uint32_t *comb_point;  // shared point g -> point number
   const uint32_t *comb_base;   // shared point g -> its slots [base[g], base[g+1])
   uint32_t n_slots, n_shared;
   const uint4 *tile_hdr;       // per tile (launch order): start, cells | colours << 16,
                                // written points, its record's offset in
-                               // units of 16 bytes (direct form)
-  // per launch: tiles run (0: combine only), the buffer they fill, whether
-  // the other buffer (previous iteration) is combined, CTAs doing that
-  uint32_t tiles_on, put_buf, comb_on, comb_ctas;
+                               // units of 16 bytes (DirectRecord)
+  // per launch: tiles run (0: combine only), the buffer they fill, CTAs
+  // combining the other buffer (previous iteration)
+  uint32_t tiles_on, put_buf, comb_ctas;
 };
 
 // Direct (cell) data of one cell: SOA with stride n_cells.

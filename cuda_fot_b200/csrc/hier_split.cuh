@@ -1,10 +1,10 @@
-// The split write-back hierarchical-colour kernels (variant kVariantSplit).
+// The split write-back hierarchical-colour kernel (variant kVariantSplit).
 //
 // The coloured replay of a plan (blocks in block-colour order; in a block,
 // cells in thread-colour order accumulate into a zeroed per-block sum; then
 // out[p] += sum for each written point) fixes, for every point p, the order
 // out[p] = ((out[p] + S_b1) + S_b2) + ... over the blocks b1 < b2 < ... (plan
-// order) that write p.  These kernels reproduce that order without making
+// order) that write p.  The kernel reproduces that order without making
 // any tile wait for another:
 //   * a point written by ONE block (private) gets out[p] += S_b as soon as
 //     the block's sum is ready -- a fire-and-forget L2 reduction (RED.F64) for
@@ -24,23 +24,14 @@
 // complete and only then write.  Loops that write cell data wait before
 // computing.
 //
-// Two forms:
-//   * k_hier_dsplit (direct): one CTA per tile, one thread per cell; each
-//     thread gathers its cell's rows straight from HBM/L2 through the
-//     plan-ordered mapping (like the atomic executor: thousands of
-//     independent gathers in flight per SM), adds its increments into a
-//     shared-memory sum one thread colour after another, and the block's
-//     sums go out as above.  Extra CTAs at the end of the grid do the
-//     combine.
-//   * k_hier_split (staged): persistent CTAs of T compute threads and two
-//     control warps; the RECORD warp bulk-copies each tile's record (plan.cu,
-//     step 4b) into one of kRecSlots slots (TMA engine, no multicast), the
-//     STAGING warp gathers the tile's read rows into one of two row slots
-//     with cp.async, the compute threads compute from shared memory.  Tile i
-//     of CTA c is launch[c + i * gridDim.x]; every CTA's compute threads
-//     combine one chunk of the shared points after their wait.  Every wait
-//     between the roles is bounded (about two seconds); on a timeout the
-//     kernel sets kErrWaitLimit in Ctl::error and returns.
+// One CTA runs one tile (k_hier_dsplit); extra CTAs at the end of the grid do
+// the combine.  A warp-specialised persistent form that staged each tile's
+// read rows in shared memory (a record warp, a staging warp, two tiles in
+// flight) was slower on every loop, layout and ordering once this one summed
+// its contributions from lists, and is gone: parts of 256, staged and direct,
+// AOS: res_calc 1000^2 60.0 and 54.7 us, LULESH 96^3 113.9 and 87.2, volna 1024^2
+// 99.7 and 53.8, getacc 1024^2 77.2 and 52.6, miniAero 96^3 634 and 413;
+// LULESH 45^3 16.7 and 11.1.
 #pragma once
 
 #include <cstdint>
@@ -61,7 +52,7 @@ __device__ __forceinline__ void griddep_wait() {
   asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
-// A tile's write-back data in the direct form (built by plan.cu): the written
+// A tile's write-back data (built by plan.cu): the written
 // points, their slots (0xFFFFFFFF: private), and per point its contributions
 // pc_idx[pc_off[j], pc_off[j + 1]) = slot * threads + cell, in thread-colour
 // order.
@@ -259,7 +250,7 @@ __device__ __forceinline__ void split_writeback(const LoopData &d, const HierPla
   }
 }
 
-// Direct form: CTAs [0, n_blocks) run one tile each, the comb_ctas after
+// CTAs [0, n_blocks) run one tile each, the comb_ctas after
 // them combine the previous buffer (hardware CTA scheduling keeps several tiles per SM in
 // different phases; a persistent form with one tile in flight per CTA and
 // the next tile's plan data prefetched measured slower).  One thread per cell
@@ -290,11 +281,9 @@ __global__ void __launch_bounds__(T, dsplit_min_blocks<L, T>()) k_hier_dsplit(Lo
     // the combine CTAs come last, so that the tiles are scheduled first
     // (they gather and compute before their wait; these only wait)
     griddep_wait();
-    if (P.comb_on) {
-      uint32_t g0, g1;
-      comb_chunk(P.n_shared, blockIdx.x - n_tiles, P.comb_ctas, g0, g1);
-      combine_shared<L, SOA>(d, P, g0, g1, tid, T);
-    }
+    uint32_t g0, g1;
+    comb_chunk(P.n_shared, blockIdx.x - n_tiles, P.comb_ctas, g0, g1);
+    combine_shared<L, SOA>(d, P, g0, g1, tid, T);
     return;
   }
   const uint4 h = __ldg(P.tile_hdr + blockIdx.x);
@@ -330,174 +319,6 @@ __global__ void __launch_bounds__(T, dsplit_min_blocks<L, T>()) k_hier_dsplit(Lo
   if constexpr (!L::kWritesCell) griddep_wait();  // the previous iteration's writes are visible
   const DirectRecord m(smem, n0);
   split_writeback<L, SOA, T>(d, P, n0, m.pts, m.wslot, m.pc_off, m.pc_idx, inc, tid);
-}
-
-template <class L, bool SOA, int T, uint32_t kRecSlots>
-__global__ void __launch_bounds__(T + 64) __maxnreg__(L::kRegCap)
-    k_hier_split(LoopData d, HierPlanDev P) {
-  using out_t = typename L::out_t;
-  using read_t = typename L::read_t;
-  constexpr int D = L::kDim, K = L::kOut;
-  constexpr uint32_t kRecordWarp = T / 32, kStagingWarp = T / 32 + 1;
-  extern __shared__ __align__(128) unsigned char smem[];
-  __shared__ __align__(8) uint64_t s_rec_full[kRecSlots];
-  __shared__ __align__(8) uint64_t s_tile_done[kRecSlots];
-  __shared__ __align__(8) uint64_t s_rows_full[2];
-  __shared__ __align__(8) uint64_t s_rows_empty[2];
-  __shared__ uint32_t s_valid[kRecSlots];  // 0: no tile (end of this CTA's tiles)
-  __shared__ volatile uint32_t s_stop;     // a role gave up (error path)
-  const uint32_t tid = threadIdx.x;
-  const uint32_t warp = tid >> 5, lane = tid & 31u;
-  unsigned char *const rec_base = smem;
-  unsigned char *const rows_base = smem + P.rows_off;
-  out_t *const inc = reinterpret_cast<out_t *>(smem + P.inc_off);
-
-  griddep_launch_dependents();
-  if (tid == 0) {
-    for (uint32_t s = 0; s < kRecSlots; ++s) {
-      mbar_init(&s_rec_full[s], 1);
-      mbar_init(&s_tile_done[s], T / 32);
-    }
-    for (int b = 0; b < 2; ++b) {
-      mbar_init(&s_rows_full[b], 33);
-      mbar_init(&s_rows_empty[b], 1);
-    }
-    mbar_fence_init();
-    s_stop = 0;
-  }
-  __syncthreads();
-
-  if (warp == kRecordWarp) {
-    // ---------------------------------------------------------------- record
-    if (lane == 0) {
-      uint32_t uses[kRecSlots] = {};
-      bool valid[kRecSlots] = {};
-      auto refill = [&](uint32_t s, uint32_t i) {
-        const uint32_t t = blockIdx.x + i * gridDim.x;
-        const bool ok = t < P.n_blocks;
-        s_valid[s] = ok;
-        valid[s] = ok;
-        if (ok) {
-          const uint32_t b = P.launch[t];
-          const uint32_t off = P.rec_off[b], end = P.rec_off[b + 1];
-          // the slot was last read through the generic proxy
-          asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-          mbar_expect_tx(&s_rec_full[s], end - off);
-          bulk_copy_g2s(rec_base + s * P.rec_slot, P.rec + off, end - off, &s_rec_full[s]);
-        } else {
-          mbar_arrive(&s_rec_full[s]);
-        }
-        ++uses[s];
-      };
-      for (uint32_t s = 0; s < kRecSlots; ++s) refill(s, s);
-      for (uint32_t i = 0;; ++i) {
-        const uint32_t s = i % kRecSlots;
-        if (!valid[s]) break;
-        if (!mbar_wait_or_stop(&s_tile_done[s], (i / kRecSlots) & 1u, &s_stop)) {
-          atomicOr(&P.ctl->error, kErrWaitLimit);
-          s_stop = 1;
-          break;
-        }
-        refill(s, i + kRecSlots);
-      }
-      // let every record copy still in flight land (bounded)
-      for (uint32_t s = 0; s < kRecSlots; ++s)
-        if (uses[s] > 0) (void)mbar_wait(&s_rec_full[s], (uses[s] - 1) & 1u);
-    }
-    __syncwarp();
-  } else if (warp == kStagingWarp) {
-    // --------------------------------------------------------------- staging
-    for (uint32_t i = 0;; ++i) {
-      const uint32_t s = i % kRecSlots, b = i & 1u;
-      bool ok = mbar_wait_or_stop(&s_rec_full[s], (i / kRecSlots) & 1u, &s_stop);
-      // the row slot of tile i - 2 is free once that tile's compute phase ended
-      if (ok && i >= 2) ok = mbar_wait_or_stop(&s_rows_empty[b], ((i - 2) >> 1) & 1u, &s_stop);
-      ok = __all_sync(0xFFFFFFFFu, ok);
-      if (!ok || !s_valid[s]) {
-        if (lane == 0) {
-          if (!ok) {
-            atomicOr(&P.ctl->error, kErrWaitLimit);
-            s_stop = 1;
-          }
-          s_valid[s] = 0;
-          mbar_arrive(&s_rows_full[b]);
-        }
-        mbar_arrive(&s_rows_full[b]);
-        break;
-      }
-      const RecView<L> m(rec_base + s * P.rec_slot);
-      ws_stage_rows<L, SOA>(d, P, rows_base + b * P.rows_bytes, m);
-      mbar_arrive_cp_async(&s_rows_full[b]);
-      if (lane == 0) mbar_arrive(&s_rows_full[b]);
-    }
-    cp_async_wait_all();
-  } else {
-    // --------------------------------------------------------------- compute
-    bool waited = false;    // griddepcontrol.wait done
-    bool combined = false;  // this CTA's combine chunk done
-    for (uint32_t i = 0;; ++i) {
-      const uint32_t s = i % kRecSlots, b = i & 1u, ph = (i >> 1) & 1u;
-      const bool ok_rows = mbar_wait_or_stop(&s_rows_full[b], ph, &s_stop);
-      if (!named_bar_and<T>(ok_rows)) {
-        if (tid == 0) {
-          atomicOr(&P.ctl->error, kErrWaitLimit);
-          s_stop = 1;
-        }
-        break;
-      }
-      if (!s_valid[s]) break;
-      // the record landed through the async proxy
-      (void)mbar_try_wait(&s_rec_full[s], (i / kRecSlots) & 1u);
-      const RecView<L> m(rec_base + s * P.rec_slot);
-      const unsigned char *rows = rows_base + b * P.rows_bytes;
-      if constexpr (L::kWritesCell) {
-        // the previous iteration may still write these cells' data
-        if (!waited) {
-          griddep_wait();
-          waited = true;
-        }
-      }
-      if (tid < m.ncell) {
-        SmemRows<L> rv;
-#pragma unroll
-        for (int q = 0; q < D; ++q) {
-          rv.l[0][q] = m.lidx0[q * m.ncell + tid];
-          rv.l[1][q] = L::kHasClass1 ? m.lidx1[q * m.ncell + tid] : 0;
-        }
-        static_for_read<L>([&](auto r) {
-          constexpr int R = decltype(r)::value;
-          rv.base[R] = reinterpret_cast<const read_t *>(rows + P.read_off[R]);
-        });
-        out_t v[D][K];
-        Direct dir{d.cell, m.start + tid, d.n_cells};
-        L::cell(rv, dir, v);
-        put_increments<L, SOA, T>(inc, v, tid);
-      }
-      named_bar_sync<T>();
-      if (tid == 0) mbar_arrive(&s_rows_empty[b]);  // the row slot may be refilled
-      if (!waited) {
-        // the previous iteration's writes must be complete and visible
-        griddep_wait();
-        waited = true;
-      }
-      if (!combined) {
-        // this CTA's share of the previous buffer's shared points
-        combined = true;
-        if (P.comb_on) {
-          uint32_t g0, g1;
-          comb_chunk(P.n_shared, blockIdx.x, gridDim.x, g0, g1);
-          combine_shared<L, SOA>(d, P, g0, g1, tid, T);
-        }
-      }
-      split_writeback<L, SOA, T>(d, P, m.n0, m.pts0, m.dep /* split plans: the slot list */, m.pc_off,
-                                 m.pc_idx, inc, tid);
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&s_tile_done[s]);
-      // the increments buffer is reused by the next tile
-      named_bar_sync<T>();
-    }
-  }
-  __syncthreads();
 }
 
 } // namespace fot

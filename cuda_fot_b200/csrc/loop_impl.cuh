@@ -43,15 +43,6 @@ template <bool SOA, uint32_t SLOTS> const void *pipe_kernel(uint32_t threads) {
   return nullptr;
 }
 
-template <bool SOA, uint32_t SLOTS> const void *split_kernel(uint32_t threads) {
-  switch (threads) {
-  case 128: return reinterpret_cast<const void *>(&k_hier_split<L, SOA, 128, SLOTS>);
-  case 256: return reinterpret_cast<const void *>(&k_hier_split<L, SOA, 256, SLOTS>);
-  case 512: return reinterpret_cast<const void *>(&k_hier_split<L, SOA, 512, SLOTS>);
-  }
-  return nullptr;
-}
-
 template <bool SOA> const void *dsplit_kernel(uint32_t threads) {
   switch (threads) {
   case 128: return reinterpret_cast<const void *>(&k_hier_dsplit<L, SOA, 128>);
@@ -62,16 +53,11 @@ template <bool SOA> const void *dsplit_kernel(uint32_t threads) {
 }
 
 // variant: kVariantStage (staged reads), kVariantPipe (pipelined kernel),
-// kVariantSplit (split write-back kernels: staged with kVariantPipe, else
-// direct)
+// kVariantSplit (split write-back kernel)
 const void *kernel_for(int exec, bool soa, uint32_t threads, uint32_t variant) {
   if (exec == FOT_EXEC_ATOMIC) return nullptr;
-  if (exec == FOT_EXEC_HIER && (variant & kVariantSplit) && !(variant & kVariantPipe))
+  if (exec == FOT_EXEC_HIER && (variant & kVariantSplit))
     return soa ? dsplit_kernel<true>(threads) : dsplit_kernel<false>(threads);
-  if (exec == FOT_EXEC_HIER && (variant & kVariantSplit)) {
-    if (variant & kVariantSlots3) return soa ? split_kernel<true, 3>(threads) : split_kernel<false, 3>(threads);
-    return soa ? split_kernel<true, 2>(threads) : split_kernel<false, 2>(threads);
-  }
   if (exec == FOT_EXEC_HIER && (variant & kVariantPipe)) {
     if (variant & kVariantSlots3) return soa ? pipe_kernel<true, 3>(threads) : pipe_kernel<false, 3>(threads);
     return soa ? pipe_kernel<true, 2>(threads) : pipe_kernel<false, 2>(threads);
@@ -98,17 +84,14 @@ int run_hier(const LoopData &d, const HierPlanDev &P, bool soa, uint32_t threads
   const uint32_t block = (variant & kVariantPipe) ? threads + 64 : threads;
   if (variant & kVariantSplit) {
     // One launch per iteration.  Launch `it` fills partial buffer it & 1 and
-    // combines buffer (it - 1) & 1 (direct form: in comb_ctas extra CTAs;
-    // staged form: in every CTA after its wait); a last, combine-only launch
-    // of the direct kernel flushes the final iteration's buffer.  From the
+    // combines buffer (it - 1) & 1 in comb_ctas extra CTAs; a last,
+    // combine-only launch flushes the final iteration's buffer.  From the
     // second launch on, programmatic dependent launch lets the next grid
-    // gather and compute while this one drains (the kernels wait before
-    // they write); the first launch of a call is fully stream-ordered:
+    // gather and compute while this one drains (the kernel waits before
+    // it writes); the first launch of a call is fully stream-ordered:
     // whatever precedes it may write the datasets it reads.
     const uint32_t iters = P.n_blocks ? P.total_tiles / P.n_blocks : 0;
-    const bool direct = !(variant & kVariantPipe);
     const uint32_t comb_ctas = (P.n_shared + threads - 1) / threads;  // a point a thread
-    const void *flush = soa ? dsplit_kernel<true>(threads) : dsplit_kernel<false>(threads);
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
@@ -121,14 +104,13 @@ int run_hier(const LoopData &d, const HierPlanDev &P, bool soa, uint32_t threads
       if (last && P.n_shared == 0) break;
       Q.tiles_on = last ? 0u : 1u;
       Q.put_buf = it & 1u;
-      Q.comb_on = it > 0 && P.n_shared > 0;
-      Q.comb_ctas = (direct || last) && Q.comb_on ? comb_ctas : 0u;
-      cfg.gridDim = dim3(last ? Q.comb_ctas : grid + (direct ? Q.comb_ctas : 0u));
-      cfg.blockDim = dim3(last ? threads : block);
+      Q.comb_ctas = it > 0 ? comb_ctas : 0u;
+      cfg.gridDim = dim3(Q.comb_ctas + (last ? 0u : grid));
+      cfg.blockDim = dim3(threads);
       cfg.dynamicSmemBytes = last ? 0 : smem;
       cfg.attrs = it > 0 ? attr : nullptr;
       cfg.numAttrs = it > 0 ? 1 : 0;
-      FOT_CUDA(cudaLaunchKernelExC(&cfg, last ? flush : k, qargs));
+      FOT_CUDA(cudaLaunchKernelExC(&cfg, k, qargs));
     }
     return FOT_OK;
   }
@@ -168,8 +150,8 @@ void smem_layout(uint32_t cap0, uint32_t cap1, uint32_t variant, uint32_t rec_ca
   auto a16 = [](size_t v) { return (v + 15) & ~size_t(15); };
   SmemLayout s;
   size_t off = 0;
-  if ((variant & kVariantSplit) && !(variant & kVariantPipe)) {
-    // direct split write-back: the tile's record and the increments
+  if (variant & kVariantSplit) {
+    // split write-back: the tile's record and the increments
     s.rec_slot = rec_cap;
     s.inc_off = (uint32_t)((rec_cap + 127u) & ~127u);
     s.total = s.inc_off + (size_t)L::kOut * L::kDim * threads * sizeof(out_t);
@@ -178,8 +160,7 @@ void smem_layout(uint32_t cap0, uint32_t cap1, uint32_t variant, uint32_t rec_ca
   }
   if (variant & kVariantPipe) {
     // 2 or 3 tile-record slots, 2 read-row slots, the per-slot increments, 2
-    // prefetched-output-row slots (AOS output rows of a multiple of 16 bytes;
-    // not in the split write-back kernel)
+    // prefetched-output-row slots (AOS output rows of a multiple of 16 bytes)
     auto a128 = [](size_t v) { return (v + 127) & ~size_t(127); };
     s.rec_slot = (uint32_t)a128(rec_cap);
     off = ((variant & kVariantSlots3) ? 3 : 2) * (size_t)s.rec_slot;
@@ -195,7 +176,7 @@ void smem_layout(uint32_t cap0, uint32_t cap1, uint32_t variant, uint32_t rec_ca
     s.inc_off = (uint32_t)off;
     off = a128(off + (size_t)L::kOut * L::kDim * threads * sizeof(out_t));
     s.outbuf_off = (uint32_t)off;
-    if (!(variant & kVariantSplit) && (L::kOut * sizeof(out_t)) % 16 == 0) {
+    if ((L::kOut * sizeof(out_t)) % 16 == 0) {
       s.outbuf_bytes = (uint32_t)a128((size_t)cap0 * L::kOut * sizeof(out_t));
       off += 2 * (size_t)s.outbuf_bytes;
     }

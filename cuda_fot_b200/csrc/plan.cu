@@ -294,16 +294,13 @@ __global__ void k_gather_plan(GatherArgs g) {
 // accumulation (res_calc.hpp:328-339).
 // dep lists the blocks sharing a written point with this one (the conflict
 // graph); bit 31 marks those of an earlier block colour.
-// Plans of the split write-back kernels (hier_split.cuh) have no dep list;
-// in its place, at the same offset, comes u32 wslot[n0] (build_split below),
-// then zero padding to 16 bytes.
+// Plans of the split write-back kernel have DirectRecords instead (below).
 // ---------------------------------------------------------------------------
 struct RecordArgs {
   const uint32_t *block_start, *block_wait, *pts_off[2], *pts[2], *rec_off;
   const uint16_t *lidx[2];
   const uint8_t *ntcol;
   const uint32_t *dep_off, *dep;
-  const uint32_t *wslot;           // split plans: per written point (pts_off order), or null
   unsigned char *rec;
   uint32_t n_cells, threads;
   int n_class, D;
@@ -377,18 +374,12 @@ __global__ void k_build_records(RecordArgs a) {
     r[i] = 0;
   uint32_t *dep = reinterpret_cast<uint32_t *>(r + dep_at);
   for (uint32_t i = threadIdx.x; i < ndep; i += blockDim.x) dep[i] = a.dep[a.dep_off[b] + i];
-  uint32_t used = dep_at + 4 * ndep;
-  if (a.wslot) {
-    uint32_t *w = reinterpret_cast<uint32_t *>(r + used);
-    const uint32_t *src = a.wslot + a.pts_off[0][b];
-    for (uint32_t i = threadIdx.x; i < n[0]; i += blockDim.x) w[i] = src[i];
-    used += 4 * n[0];
-  }
+  const uint32_t used = dep_at + 4 * ndep;
   for (uint32_t i = used + threadIdx.x; i < a.rec_off[b + 1] - a.rec_off[b]; i += blockDim.x) r[i] = 0;
 }
 
-// The direct form's records (DirectRecord, hier_split.cuh): the same lists
-// without what only the staged form reads.  Cells of one thread colour write
+// The split write-back kernel's records (DirectRecord, hier_split.cuh): the
+// contribution lists with the points and their slots.  Cells of one thread colour write
 // disjoint points, so that, colour by colour, each cell appends its entries to
 // its points' lists: one step per colour instead of a scan of all entries per
 // point.
@@ -759,7 +750,6 @@ int build_hier_plan(fot_problem *p, fot_plan *plan) {
   // 4b. tile records
   {
     const bool split = plan->variant & kVariantSplit;
-    const bool direct = split && !(plan->variant & kVariantPipe);
     std::vector<uint32_t> final_of(nfb);
     for (uint32_t b = 0; b < nfb; ++b) final_of[order[b]] = b;
     // conflict neighbours of each block in final order; bit 31: earlier
@@ -790,14 +780,12 @@ int build_hier_plan(fot_problem *p, fot_plan *plan) {
       FOT_TRY(plan->partial.alloc(2 * (size_t)sr.n_slots * row));
       FOT_TRY(upload(plan->comb_point, sr.point));
       FOT_TRY(upload(plan->comb_base, sr.base));
-      FOT_TRY(upload(plan->launch, final_of));
-      // direct form: one 16-byte header per tile, in launch order
       std::vector<uint32_t> drec_off(nfb + 1, 0);  // direct records, in units of 16 bytes
       for (uint32_t b = 0; b < nfb; ++b) {
         const uint32_t bytes = DirectRecord::bytes(h_off[0][b + 1] - h_off[0][b],
                                                    D * (block_start[b + 1] - block_start[b]));
         drec_off[b + 1] = drec_off[b] + bytes / 16;
-        if (direct) plan->rec_cap = std::max(plan->rec_cap, bytes);
+        plan->rec_cap = std::max(plan->rec_cap, bytes);
       }
       std::vector<uint32_t> hdr((size_t)4 * nfb);
       for (uint32_t t = 0; t < nfb; ++t) {
@@ -808,40 +796,37 @@ int build_hier_plan(fot_problem *p, fot_plan *plan) {
         hdr[4 * t + 3] = drec_off[b];
       }
       FOT_TRY(upload(plan->tile_hdr, hdr));
-      if (direct) {
-        std::vector<uint32_t> first(nfb);
-        for (uint32_t t = 0; t < nfb; ++t) first[t] = h_off[0][final_of[t]];
-        FOT_TRY(upload(d_first, first));
-        FOT_TRY(plan->rec.alloc((size_t)drec_off[nfb] * 16));
-        DirectRecordArgs da{};
-        da.hdr = plan->tile_hdr.as<uint4>();
-        da.pts_first = d_first.as<uint32_t>();
-        da.pts = plan->pts[0].as<uint32_t>();
-        da.wslot = d_split.as<uint32_t>();
-        da.lidx = plan->lidx[0].as<uint16_t>();
-        da.tcol = plan->tcol.as<uint8_t>();
-        da.rec = plan->rec.as<unsigned char>();
-        da.n_cells = n;
-        da.threads = hier_threads(B);
-        da.D = D;
-        k_build_direct_records<<<nfb, 128, (plan->cap[0] + 1) * sizeof(uint32_t)>>>(da);
-        FOT_CUDA(cudaGetLastError());
-      }
+      std::vector<uint32_t> first(nfb);
+      for (uint32_t t = 0; t < nfb; ++t) first[t] = h_off[0][final_of[t]];
+      FOT_TRY(upload(d_first, first));
+      FOT_TRY(plan->rec.alloc((size_t)drec_off[nfb] * 16));
+      DirectRecordArgs da{};
+      da.hdr = plan->tile_hdr.as<uint4>();
+      da.pts_first = d_first.as<uint32_t>();
+      da.pts = plan->pts[0].as<uint32_t>();
+      da.wslot = d_split.as<uint32_t>();
+      da.lidx = plan->lidx[0].as<uint16_t>();
+      da.tcol = plan->tcol.as<uint8_t>();
+      da.rec = plan->rec.as<unsigned char>();
+      da.n_cells = n;
+      da.threads = hier_threads(B);
+      da.D = D;
+      k_build_direct_records<<<nfb, 128, (plan->cap[0] + 1) * sizeof(uint32_t)>>>(da);
+      FOT_CUDA(cudaGetLastError());
       plan->n_slots = sr.n_slots;
       plan->n_shared_points = (uint32_t)sr.point.size();
     }
     // completed iterations of each block (the dependency flags)
     FOT_TRY(plan->block_done.alloc((size_t)nfb * 4));
     FOT_CUDA(cudaMemset(plan->block_done.ptr, 0, (size_t)nfb * 4));
-    if (!direct) {
+    if (!split) {
       std::vector<uint32_t> rec_off(nfb + 1, 0);
       uint32_t rec_cap = 0;
       for (uint32_t b = 0; b < nfb; ++b) {
         const uint32_t ncell = block_start[b + 1] - block_start[b];
         const uint32_t n0 = h_off[0][b + 1] - h_off[0][b];
         const uint32_t n1 = n_class > 1 ? h_off[1][b + 1] - h_off[1][b] : 0;
-        uint32_t padded = record_bytes(ncell, n0, n1, D, n_class, dep_off[b + 1] - dep_off[b]);
-        if (split) padded = (record_dep_offset(ncell, n0, n1, D, n_class) + 4 * n0 + 15) & ~15u;
+        const uint32_t padded = record_bytes(ncell, n0, n1, D, n_class, dep_off[b + 1] - dep_off[b]);
         rec_cap = std::max(rec_cap, padded);
         rec_off[b + 1] = rec_off[b] + padded;
       }
@@ -855,7 +840,6 @@ int build_hier_plan(fot_problem *p, fot_plan *plan) {
       ra.threads = hier_threads(B);
       ra.dep_off = d_dep_off.as<uint32_t>();
       ra.dep = d_dep.as<uint32_t>();
-      ra.wslot = split ? d_split.as<uint32_t>() : nullptr;
       ra.ntcol = plan->block_ntcol.as<uint8_t>();
       ra.rec = plan->rec.as<unsigned char>();
       ra.n_cells = n;

@@ -74,18 +74,20 @@ extern "C" {
 /* plan flags */
 #define FOT_PLAN_NO_AGGREGATE 1u /* atomic executor: no warp aggregation */
 #define FOT_PLAN_USE_PARTITION 2u /* hierarchical: blocks from the partition */
-#define FOT_PLAN_DIRECT_READS 4u  /* hierarchical: gather read rows from HBM/L2 instead of
-                                     staging them in shared memory (persistent executor:
-                                     the direct split write-back kernel, one CTA per block) */
+#define FOT_PLAN_DIRECT_READS 4u  /* hierarchical, simple tiles and per-colour launches: gather
+                                     read rows from HBM/L2 instead of staging them in shared
+                                     memory (the default split write-back kernel always
+                                     does) */
 #define FOT_PLAN_SIMPLE_TILES 8u  /* persistent hierarchical: one tile at a time with a
                                      barrier per thread colour (no pipelining) */
 #define FOT_PLAN_BLOCK_FLAGS 16u  /* persistent hierarchical: the pipelined kernel whose tiles
                                      wait for the per-block completion flags of the blocks
                                      they conflict with, all iterations in one launch (the
-                                     default is the split write-back kernel: no tile waits,
-                                     points shared by several blocks are summed in colour
-                                     order by the next launch, one launch per iteration
-                                     and a combine-only launch at the end of a call) */
+                                     default is the split write-back kernel, one CTA per
+                                     block: no tile waits, points shared by several blocks
+                                     are summed in colour order by the next launch, one
+                                     launch per iteration and a combine-only launch at the
+                                     end of a call) */
 
 typedef struct fot_problem fot_problem;
 typedef struct fot_plan fot_plan;
