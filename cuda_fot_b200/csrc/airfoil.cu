@@ -22,9 +22,13 @@
 // cell -> 4 nodes, boundary edge -> 2 nodes / 1 cell / bound flag (given in
 // the original numbering and renumbered here whenever the problem's
 // numbering changes).  The per-cell loops run fused, each cell's values
-// unchanged: update + the next stage's adt_calc in one pass (and between
-// iterations + save_soln), so an iteration is two res_calc runs, two
-// bres_calc launches, two cell passes and the rms reduction.
+// unchanged: bres_calc + update + the next stage's adt_calc in one pass (and
+// between iterations + save_soln), whose last CTA sums the rms: an iteration
+// is two res_calc runs and two cell passes.  bres_calc (4 edges of a cell at
+// most, here) and the rms as launches of their own were 3 of 7 launches an
+// iteration, each a few us of start and drain for next to no work: 185 us
+// an iteration of 1000^2 so (169 us as a graph), 173 us fused (165); 300^2 42 and
+// 28.5 us (28.4 and 21.8).
 // Every kernel is compiled without multiply-add
 // contraction, and every sum has a fixed order: boundary edges are added per
 // cell in increasing edge order (one thread per boundary cell), the rms is a
@@ -45,6 +49,13 @@ constexpr uint32_t kThreads = 256;
 #ifndef FOT_AIRFOIL_MAX_CTAS
 #define FOT_AIRFOIL_MAX_CTAS 1184
 #endif
+#ifndef FOT_CELLS_MINB
+#define FOT_CELLS_MINB 4
+#endif
+// resident CTAs per SM of a cell pass: the boundary branch needs 62 registers;
+// 5 CTAs spill in it (1000^2 173 us an iteration with 4 and with 5, 176 with 6, 184
+// with 8; AOS 200, 204, 221, 226)
+constexpr int kCellsMinCtas = FOT_CELLS_MINB;
 // CTAs of a cell pass (grid-stride beyond); the rms sums one partial per CTA
 constexpr uint32_t kMaxUpdateCtas = FOT_AIRFOIL_MAX_CTAS;
 
@@ -54,11 +65,14 @@ struct AirfoilDev {
   uint32_t n_nodes, n_cells;
   int soa;
   const uint4 *cell_nodes;      // per cell: its 4 nodes, counter-clockwise
-  const uint32_t *bcell;        // boundary cells
-  const uint32_t *bcell_off;    // their boundary edges [off[i], off[i+1]) in bedge order
+  // boundary cells: bit c & 31 of boundary[c / 32] is set, the cell's rank i
+  // among them is before[c / 32] plus the set bits below
+  const uint32_t *boundary, *before;
+  const uint32_t *bcell_off;    // edges [off[i], off[i+1]) of boundary cell i in bedge order
   const uint2 *bedge_nodes;     // per boundary edge (grouped by cell): node 1, node 2
   const int *bedge_bound;       // 1: solid wall, else far field
-  uint32_t n_bcells;
+  unsigned int *arrived;        // CTAs of a pass that wrote their partial sum
+  double *rms;
   double qinf[4];
   double cfl;
 };
@@ -90,18 +104,10 @@ __device__ __forceinline__ double cell_adt(const AirfoilDev &a, uint32_t c, cons
   return s / a.cfl;
 }
 
-// One thread per boundary cell: its boundary edges in increasing edge order.
-__global__ void __launch_bounds__(kThreads) k_bres_calc(AirfoilDev a) {
-  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= a.n_bcells) return;
-  const uint32_t c = a.bcell[i];
-  double q[4], r[4];
-#pragma unroll
-  for (int k = 0; k < 4; ++k) {
-    q[k] = a.q[at(a.soa, a.n_cells, c, 4, k)];
-    r[k] = a.res[at(a.soa, a.n_cells, c, 4, k)];
-  }
-  const double adt1 = a.adt[c];
+// bres_calc of boundary cell i (state q, time step adt1): its boundary edges
+// added to its residual r in increasing edge order.
+__device__ __forceinline__ void add_boundary(const AirfoilDev &a, uint32_t i, const double (&q)[4],
+                                             double adt1, double (&r)[4]) {
   for (uint32_t e = a.bcell_off[i]; e < a.bcell_off[i + 1]; ++e) {
     const uint2 nd = a.bedge_nodes[e];
     const double dx = a.x[at(a.soa, a.n_nodes, nd.x, 2, 0)] - a.x[at(a.soa, a.n_nodes, nd.y, 2, 0)];
@@ -124,8 +130,6 @@ __global__ void __launch_bounds__(kThreads) k_bres_calc(AirfoilDev a) {
       r[3] += 0.5 * (vol1 * (q[3] + p1) + vol2 * (qi[3] + p2)) + mu * (q[3] - qi[3]);
     }
   }
-#pragma unroll
-  for (int k = 0; k < 4; ++k) a.res[at(a.soa, a.n_cells, c, 4, k)] = r[k];
 }
 
 // Sum of the block's values in a fixed order (warp trees, then the warps'
@@ -143,26 +147,39 @@ __device__ __forceinline__ double block_sum(double v, double *smem) {
 }
 
 // The per-cell loops of the iteration, fused (each cell's values are the
-// same as loop by loop): UPDATE (q = qold - res / adt, res = 0, squared
-// updates summed per CTA in a fixed order into partial[]), then SAVE
-// (qold = q: save_soln of the next iteration) and ADT (adt_calc on the new q).
-template <bool UPDATE, bool SAVE, bool ADT>
-__global__ void __launch_bounds__(kThreads) k_cells(AirfoilDev a, double *partial) {
+// same as loop by loop): UPDATE (bres_calc where the cell has boundary edges,
+// q = qold - res / adt, res = 0), with RMS the squared updates summed per CTA
+// in a fixed order into partial[] and those by the last CTA to arrive, in CTA
+// order; then SAVE (qold = q: save_soln of the next iteration) and ADT
+// (adt_calc on the new q).
+template <bool UPDATE, bool SAVE, bool ADT, bool RMS>
+__global__ void __launch_bounds__(kThreads, kCellsMinCtas) k_cells(AirfoilDev a, double *partial) {
   __shared__ double smem[kThreads / 32];
+  __shared__ bool s_last;
   double sum = 0.0;
   const uint32_t stride = gridDim.x * blockDim.x;
   for (uint32_t c = blockIdx.x * blockDim.x + threadIdx.x; c < a.n_cells; c += stride) {
     double q[4];
     if constexpr (UPDATE) {
-      const double adti = 1.0 / a.adt[c];
+      const double adt = a.adt[c];
+      double r[4];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) r[k] = a.res[at(a.soa, a.n_cells, c, 4, k)];
+      const uint32_t word = a.boundary[c >> 5], bit = 1u << (c & 31u);
+      if (word & bit) {
+#pragma unroll
+        for (int k = 0; k < 4; ++k) q[k] = a.q[at(a.soa, a.n_cells, c, 4, k)];
+        add_boundary(a, a.before[c >> 5] + __popc(word & (bit - 1u)), q, adt, r);
+      }
+      const double adti = 1.0 / adt;
 #pragma unroll
       for (int k = 0; k < 4; ++k) {
         const size_t o = at(a.soa, a.n_cells, c, 4, k);
-        const double del = adti * a.res[o];
+        const double del = adti * r[k];
         q[k] = a.qold[o] - del;
         a.q[o] = q[k];
         a.res[o] = 0.0;
-        sum += del * del;
+        if constexpr (RMS) sum += del * del;
       }
     } else {
 #pragma unroll
@@ -174,19 +191,24 @@ __global__ void __launch_bounds__(kThreads) k_cells(AirfoilDev a, double *partia
     }
     if constexpr (ADT) a.adt[c] = cell_adt(a, c, q);
   }
-  if constexpr (UPDATE) {
+  if constexpr (RMS) {
     const double s = block_sum(sum, smem);
-    if (threadIdx.x == 0) partial[blockIdx.x] = s;
+    if (threadIdx.x == 0) {
+      partial[blockIdx.x] = s;
+      __threadfence();
+      s_last = atomicAdd(a.arrived, 1u) == gridDim.x - 1;
+    }
+    __syncthreads();
+    if (!s_last) return;
+    __threadfence();
+    double v = 0.0;
+    for (uint32_t i = threadIdx.x; i < gridDim.x; i += blockDim.x) v += __ldcg(partial + i);
+    const double all = block_sum(v, smem);
+    if (threadIdx.x == 0) {
+      *a.rms = sqrt(all / (double)a.n_cells);
+      *a.arrived = 0;
+    }
   }
-}
-
-__global__ void __launch_bounds__(kThreads) k_rms(const double *partial, uint32_t n_partial,
-                                                 uint32_t n_cells, double *rms) {
-  __shared__ double smem[kThreads / 32];
-  double v = 0.0;
-  for (uint32_t i = threadIdx.x; i < n_partial; i += blockDim.x) v += partial[i];
-  const double s = block_sum(v, smem);
-  if (threadIdx.x == 0) *rms = sqrt(s / (double)n_cells);
 }
 
 uint32_t update_ctas(uint32_t n_cells) {
@@ -208,9 +230,8 @@ struct fot_airfoil {
   double qinf[4] = {0, 0, 0, 0};
   double cfl = 0.0;
   // device, current numbering
-  DevBuf d_cell_nodes, d_bcell, d_bcell_off, d_bedge_nodes, d_bedge_bound;
-  uint32_t n_bcells = 0;
-  DevBuf qold, partial, rms;
+  DevBuf d_cell_nodes, d_boundary, d_before, d_bcell_off, d_bedge_nodes, d_bedge_bound;
+  DevBuf qold, partial, rms, arrived;
 };
 
 namespace {
@@ -249,9 +270,13 @@ int airfoil_renumber(fot_airfoil *a) {
     bb[i] = a->bound[e];
   }
   boff.push_back(a->n_bedges);
-  a->n_bcells = (uint32_t)bcell.size();
+  std::vector<uint32_t> boundary((a->n_cells + 31) / 32, 0), before(boundary.size(), 0);
+  for (uint32_t c : bcell) boundary[c >> 5] |= 1u << (c & 31u);
+  for (size_t w = 1; w < boundary.size(); ++w)
+    before[w] = before[w - 1] + (uint32_t)__builtin_popcount(boundary[w - 1]);
   FOT_TRY(upload(a->d_cell_nodes, cn.data(), cn.size() * sizeof(uint32_t)));
-  FOT_TRY(upload(a->d_bcell, bcell.data(), bcell.size() * sizeof(uint32_t)));
+  FOT_TRY(upload(a->d_boundary, boundary.data(), boundary.size() * sizeof(uint32_t)));
+  FOT_TRY(upload(a->d_before, before.data(), before.size() * sizeof(uint32_t)));
   FOT_TRY(upload(a->d_bcell_off, boff.data(), boff.size() * sizeof(uint32_t)));
   FOT_TRY(upload(a->d_bedge_nodes, bnodes.data(), bnodes.size() * sizeof(uint32_t)));
   FOT_TRY(upload(a->d_bedge_bound, bb.data(), bb.size() * sizeof(int32_t)));
@@ -297,7 +322,9 @@ int fot_airfoil_create(fot_problem *p, const fot_airfoil_desc *desc, fot_airfoil
   if (rc == FOT_OK) rc = a->qold.alloc((size_t)n_cells * 4 * sizeof(double));
   if (rc == FOT_OK) rc = a->partial.alloc(update_ctas(n_cells) * sizeof(double));
   if (rc == FOT_OK) rc = a->rms.alloc(sizeof(double));
-  if (rc == FOT_OK && cudaMemset(a->rms.ptr, 0, sizeof(double)) != cudaSuccess)
+  if (rc == FOT_OK) rc = a->arrived.alloc(sizeof(unsigned int));
+  if (rc == FOT_OK && (cudaMemset(a->rms.ptr, 0, sizeof(double)) != cudaSuccess ||
+                       cudaMemset(a->arrived.ptr, 0, sizeof(unsigned int)) != cudaSuccess))
     rc = fail(FOT_ERR_CUDA, "cudaMemset failed");
   if (rc != FOT_OK) {
     delete a;
@@ -335,37 +362,32 @@ int airfoil_enqueue(fot_airfoil *a, fot_plan *plan, uint32_t iterations, cudaStr
   d.n_cells = a->n_cells;
   d.soa = p->layout == FOT_SOA;
   d.cell_nodes = a->d_cell_nodes.as<uint4>();
-  d.bcell = a->d_bcell.as<uint32_t>();
+  d.boundary = a->d_boundary.as<uint32_t>();
+  d.before = a->d_before.as<uint32_t>();
   d.bcell_off = a->d_bcell_off.as<uint32_t>();
   d.bedge_nodes = a->d_bedge_nodes.as<uint2>();
   d.bedge_bound = a->d_bedge_bound.as<int>();
-  d.n_bcells = a->n_bcells;
+  d.arrived = a->arrived.as<unsigned int>();
+  d.rms = a->rms.as<double>();
   std::memcpy(d.qinf, a->qinf, sizeof(d.qinf));
   d.cfl = a->cfl;
   const uint32_t ctas = update_ctas(a->n_cells);
-  const uint32_t bctas = (a->n_bcells + kThreads - 1) / kThreads;
   double *part = a->partial.as<double>();
   // save_soln + adt_calc of the first stage; afterwards each update carries
   // the next stage's adt_calc (and, between iterations, save_soln)
-  k_cells<false, true, true><<<ctas, kThreads, 0, st>>>(d, part);
+  k_cells<false, true, true, false><<<ctas, kThreads, 0, st>>>(d, part);
   FOT_CUDA(cudaGetLastError());
   for (uint32_t it = 0; it < iterations; ++it) {
     for (int stage = 0; stage < 2; ++stage) {
       FOT_TRY(fot_run(p, plan, 1, st));
-      if (bctas) {
-        k_bres_calc<<<bctas, kThreads, 0, st>>>(d);
-        FOT_CUDA(cudaGetLastError());
-      }
       if (stage == 0)
-        k_cells<true, false, true><<<ctas, kThreads, 0, st>>>(d, part);
+        k_cells<true, false, true, false><<<ctas, kThreads, 0, st>>>(d, part);
       else if (it + 1 < iterations)
-        k_cells<true, true, true><<<ctas, kThreads, 0, st>>>(d, part);
+        k_cells<true, true, true, true><<<ctas, kThreads, 0, st>>>(d, part);
       else
-        k_cells<true, false, false><<<ctas, kThreads, 0, st>>>(d, part);
+        k_cells<true, false, false, true><<<ctas, kThreads, 0, st>>>(d, part);
       FOT_CUDA(cudaGetLastError());
     }
-    k_rms<<<1, kThreads, 0, st>>>(part, ctas, a->n_cells, a->rms.as<double>());
-    FOT_CUDA(cudaGetLastError());
   }
   return FOT_OK;
 }
