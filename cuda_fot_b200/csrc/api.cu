@@ -178,6 +178,64 @@ namespace fot {
 int build_hier_plan(fot_problem *p, fot_plan *plan);
 }
 
+// Remember every plan with a device control block that ran since the last
+// fot_sync, so that fot_sync reports (and clears) the device-side errors of
+// all of them, not only of the last one.
+static void note_run(fot_problem *p, fot_plan *plan) {
+  if (!plan->ctl.ptr) return;
+  if (std::find(p->pending.begin(), p->pending.end(), plan) == p->pending.end())
+    p->pending.push_back(plan);
+}
+
+namespace fot {
+
+static int enqueue_plan(fot_problem *p, fot_plan *plan, uint32_t iterations, bool backwards,
+                        cudaStream_t st) {
+  if (!p || !plan) return fail(FOT_ERR_ARG, "null argument");
+  if (plan->prob != p) return fail(FOT_ERR_STATE, "plan belongs to another (or a destroyed) problem");
+  if (iterations == 0) return FOT_OK;
+  const LoopOps *ops = loop_ops(p->loop);
+  const LoopData d = p->loop_data();
+  const bool soa = p->layout == FOT_SOA;
+  const int sms = device_sm_count();
+  if (plan->point_layout != p->layout)
+    return fail(FOT_ERR_STATE, "plan is stale: the problem's point layout changed after the plan was built");
+  if (plan->desc.exec == FOT_EXEC_ATOMIC) {
+    const bool agg = !(plan->desc.flags & FOT_PLAN_NO_AGGREGATE);
+    return ops->run_atomic(d, soa, agg, (uint32_t)(plan->per_sm * sms), iterations, backwards, st);
+  }
+  if (plan->version != p->version)
+    return fail(FOT_ERR_STATE, "plan is stale: the problem was reordered after the plan was built");
+  if (plan->desc.exec == FOT_EXEC_HIER) {
+    if ((uint64_t)iterations * plan->n_blocks + (uint64_t)plan->per_sm * sms >= 0xFFFFFFFFull)
+      return fail(FOT_ERR_LIMIT, "too many tiles in one launch");
+    const HierPlanDev P = plan->dev(iterations);
+    // the split kernel runs one iteration per launch, one CTA per block
+    const uint32_t grid = (plan->variant & kVariantSplit)
+                              ? plan->n_blocks
+                              : std::min<uint32_t>(P.total_tiles, (uint32_t)(plan->per_sm * sms));
+    return ops->run_hier(d, P, soa, plan->threads, plan->variant, grid, plan->smem, backwards, st);
+  }
+  const HierPlanDev P = plan->dev(1);
+  for (uint32_t it = 0; it < iterations; ++it)
+    for (uint32_t c = 0; c < plan->n_colours; ++c) {
+      const uint32_t first = plan->colour_offsets[c];
+      const uint32_t count = plan->colour_offsets[c + 1] - first;
+      if (count)
+        FOT_TRY(ops->run_hier_colour(d, P, soa, plan->threads, plan->variant, first, count,
+                                     plan->smem, st));
+    }
+  return FOT_OK;
+}
+
+int run_plan(fot_problem *p, fot_plan *plan, uint32_t iterations, bool backwards, cudaStream_t st) {
+  FOT_TRY(enqueue_plan(p, plan, iterations, backwards, st));
+  note_run(p, plan);
+  return FOT_OK;
+}
+
+} // namespace fot
+
 extern "C" {
 
 const char *fot_last_error(void) { return g_error.c_str(); }
@@ -516,15 +574,6 @@ int fot_plan_destroy(fot_plan *plan) {
   return FOT_OK;
 }
 
-// Remember every plan with a device control block that ran since the last
-// fot_sync, so that fot_sync reports (and clears) the device-side errors of
-// all of them, not only of the last one.
-static void note_run(fot_problem *p, fot_plan *plan) {
-  if (!plan->ctl.ptr) return;
-  if (std::find(p->pending.begin(), p->pending.end(), plan) == p->pending.end())
-    p->pending.push_back(plan);
-}
-
 int fot_plan_get_stats(const fot_plan *plan, fot_plan_stats *stats) {
   if (!plan || !stats) return fail(FOT_ERR_ARG, "null argument");
   *stats = plan->stats;
@@ -559,47 +608,8 @@ int fot_plan_export(const fot_plan *plan, uint32_t *n_blocks, uint32_t *n_colour
 
 // ---- execution ------------------------------------------------------------
 
-static int run_plan(fot_problem *p, fot_plan *plan, uint32_t iterations, cudaStream_t st) {
-  if (!p || !plan) return fail(FOT_ERR_ARG, "null argument");
-  if (plan->prob != p) return fail(FOT_ERR_STATE, "plan belongs to another (or a destroyed) problem");
-  if (iterations == 0) return FOT_OK;
-  const LoopOps *ops = loop_ops(p->loop);
-  const LoopData d = p->loop_data();
-  const bool soa = p->layout == FOT_SOA;
-  const int sms = device_sm_count();
-  if (plan->point_layout != p->layout)
-    return fail(FOT_ERR_STATE, "plan is stale: the problem's point layout changed after the plan was built");
-  if (plan->desc.exec == FOT_EXEC_ATOMIC) {
-    const bool agg = !(plan->desc.flags & FOT_PLAN_NO_AGGREGATE);
-    return ops->run_atomic(d, soa, agg, (uint32_t)(plan->per_sm * sms), iterations, st);
-  }
-  if (plan->version != p->version)
-    return fail(FOT_ERR_STATE, "plan is stale: the problem was reordered after the plan was built");
-  if (plan->desc.exec == FOT_EXEC_HIER) {
-    if ((uint64_t)iterations * plan->n_blocks + (uint64_t)plan->per_sm * sms >= 0xFFFFFFFFull)
-      return fail(FOT_ERR_LIMIT, "too many tiles in one launch");
-    const HierPlanDev P = plan->dev(iterations);
-    // the split kernel runs one iteration per launch, one CTA per block
-    const uint32_t grid = (plan->variant & kVariantSplit)
-                              ? plan->n_blocks
-                              : std::min<uint32_t>(P.total_tiles, (uint32_t)(plan->per_sm * sms));
-    return ops->run_hier(d, P, soa, plan->threads, plan->variant, grid, plan->smem, st);
-  }
-  const HierPlanDev P = plan->dev(1);
-  for (uint32_t it = 0; it < iterations; ++it)
-    for (uint32_t c = 0; c < plan->n_colours; ++c) {
-      const uint32_t first = plan->colour_offsets[c];
-      const uint32_t count = plan->colour_offsets[c + 1] - first;
-      if (count)
-        FOT_TRY(ops->run_hier_colour(d, P, soa, plan->threads, plan->variant, first, count,
-                                     plan->smem, st));
-    }
-  return FOT_OK;
-}
-
 int fot_run(fot_problem *p, fot_plan *plan, uint32_t iterations, void *stream) {
-  FOT_TRY(run_plan(p, plan, iterations, static_cast<cudaStream_t>(stream)));
-  note_run(p, plan);
+  FOT_TRY(run_plan(p, plan, iterations, false, static_cast<cudaStream_t>(stream)));
   return FOT_OK;
 }
 
@@ -649,7 +659,7 @@ int fot_graph_create(fot_problem *p, fot_plan *plan, uint32_t iterations, void *
   } ctx{p, plan, iterations};
   auto enqueue = [](void *c, cudaStream_t st) {
     const Ctx *x = static_cast<const Ctx *>(c);
-    return run_plan(x->p, x->plan, x->iterations, st);
+    return enqueue_plan(x->p, x->plan, x->iterations, false, st);
   };
   FOT_TRY(capture_graph(static_cast<cudaStream_t>(stream), enqueue, &ctx, out));
   (*out)->prob = p;

@@ -103,6 +103,33 @@ constexpr unsigned int kErrWaitLimit = 1u;
 // sleep): about 2-4 s before the kernel gives up and flags kErrWaitLimit.
 constexpr unsigned int kWaitPollLimit = 8u * 1000u * 1000u;
 
+// Programmatic dependent launch (sm_90+): let the dependent grid launch /
+// wait for the prerequisite grid to complete with its memory visible.  Both
+// are no-ops when the grid was launched without the programmatic attribute.
+__device__ __forceinline__ void griddep_launch_dependents() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+__device__ __forceinline__ void griddep_wait() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+// Host side: launch attribute of a grid that may start while the one before it
+// on the stream drains (its kernel calls griddep_wait before it touches what
+// that one writes).
+struct Chained {
+  cudaLaunchAttribute attr[1];
+  cudaLaunchConfig_t cfg = {};
+  Chained(dim3 grid, dim3 block, size_t smem, cudaStream_t st) {
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+  }
+};
+
 // ---- loop descriptions ------------------------------------------------------
 int describe(int loop, fot_loop_info *info);
 

@@ -36,12 +36,13 @@ constexpr uint32_t kVariantStage = 1u, kVariantPipe = 2u, kVariantSlots3 = 4u, k
 
 struct LoopOps {
   // launch `iterations` iterations of the atomic executor; resident: CTAs the
-  // GPU holds at once
+  // GPU holds at once; backwards: the first one runs last tile to first
   int (*run_atomic)(const LoopData &d, bool soa, bool aggregate, uint32_t resident,
-                    uint32_t iterations, cudaStream_t st);
-  // persistent hierarchical launch over P.total_tiles tiles
+                    uint32_t iterations, bool backwards, cudaStream_t st);
+  // persistent hierarchical launch over P.total_tiles tiles (backwards: split
+  // write-back kernel only)
   int (*run_hier)(const LoopData &d, const HierPlanDev &P, bool soa, uint32_t threads,
-                  uint32_t variant, uint32_t grid, size_t smem, cudaStream_t st);
+                  uint32_t variant, uint32_t grid, size_t smem, bool backwards, cudaStream_t st);
   // one launch per block colour: blocks [first, first + count)
   int (*run_hier_colour)(const LoopData &d, const HierPlanDev &P, bool soa,
                          uint32_t threads, uint32_t variant, uint32_t first, uint32_t count,
@@ -115,6 +116,10 @@ void fot_airfoil_detach(struct fot_airfoil *a);
 void fot_rowlist_detach(struct fot_rowlist *l);
 
 namespace fot {
+// fot_run, with the first iteration's direction through the mesh (results do
+// not depend on it: coloured plans fix the order of every sum, atomic plans
+// none).
+int run_plan(fot_problem *p, fot_plan *plan, uint32_t iterations, bool backwards, cudaStream_t st);
 // Capture into a new fot_graph what enqueue(ctx, stream) launches (on a
 // private non-blocking stream when st is the legacy default stream).
 int capture_graph(cudaStream_t st, int (*enqueue)(void *ctx, cudaStream_t st), void *ctx,

@@ -42,16 +42,6 @@
 
 namespace fot {
 
-// Programmatic dependent launch (sm_90+): let the dependent grid launch /
-// wait for the prerequisite grid to complete with its memory visible.  Both
-// are no-ops when the grid was launched without the programmatic attribute.
-__device__ __forceinline__ void griddep_launch_dependents() {
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-}
-__device__ __forceinline__ void griddep_wait() {
-  asm volatile("griddepcontrol.wait;" ::: "memory");
-}
-
 // A tile's write-back data (built by plan.cu): the written
 // points, their slots (0xFFFFFFFF: private), and per point its contributions
 // pc_idx[pc_off[j], pc_off[j + 1]) = slot * threads + cell, in thread-colour
@@ -276,6 +266,7 @@ __global__ void __launch_bounds__(T, dsplit_min_blocks<L, T>()) k_hier_dsplit(Lo
   out_t *const inc = reinterpret_cast<out_t *>(smem + P.inc_off);
   const uint32_t tid = threadIdx.x;
   griddep_launch_dependents();
+  if (P.ordered) griddep_wait();  // what precedes a call may write what its tiles read
   const uint32_t n_tiles = P.tiles_on ? P.n_blocks : 0u;
   if (blockIdx.x >= n_tiles) {
     // the combine CTAs come last, so that the tiles are scheduled first
@@ -286,7 +277,7 @@ __global__ void __launch_bounds__(T, dsplit_min_blocks<L, T>()) k_hier_dsplit(Lo
     combine_shared<L, SOA>(d, P, g0, g1, tid, T);
     return;
   }
-  const uint4 h = __ldg(P.tile_hdr + blockIdx.x);
+  const uint4 h = __ldg(P.tile_hdr + (P.backwards ? n_tiles - 1u - blockIdx.x : blockIdx.x));
   const uint32_t start = h.x, ncell = h.y & 0xFFFFu, n0 = h.z;
   if (tid == 0) {
     const uint32_t bytes = DirectRecord::bytes(n0, D * ncell);

@@ -24,8 +24,10 @@ using LA = FOT_LNS(FOT_ADAPTER_NS)::Loop;
 // `iterations` iterations in one launch (more only where the grid would grow
 // past 2^30 CTAs).
 template <bool SOA, bool AGG>
-int launch_atomic(const LoopData &d, uint32_t resident, uint32_t iterations, cudaStream_t st) {
+int launch_atomic(const LoopData &d, uint32_t resident, uint32_t iterations, bool backwards,
+                  cudaStream_t st) {
   AtomicGrid g;
+  g.flip = backwards;
   g.tiles = (d.n_cells + 255u) / 256u;
   g.resident = std::max(1u, std::min(g.tiles, resident));
   const uint32_t all = (g.tiles + g.resident - 1) / g.resident;
@@ -37,9 +39,10 @@ int launch_atomic(const LoopData &d, uint32_t resident, uint32_t iterations, cud
   const uint32_t most = std::max(1u, (1u << 30) / g.ctas);
   while (iterations) {
     const uint32_t now = std::min(iterations, most);
-    k_atomic<LA, SOA, AGG><<<g.ctas * now, 256, 0, st>>>(d, g);
-    FOT_CUDA(cudaGetLastError());
+    Chained c(dim3(g.ctas * now), dim3(256), 0, st);
+    FOT_CUDA(cudaLaunchKernelEx(&c.cfg, k_atomic<LA, SOA, AGG>, d, g));
     iterations -= now;
+    g.flip += now;
   }
   return FOT_OK;
 }
@@ -51,11 +54,11 @@ template <bool SOA, bool AGG> const void *atomic_kernel() {
 } // namespace
 
 int FOT_CAT(atomic_run_, FOT_ADAPTER_NS)(const LoopData &d, bool soa, bool agg, uint32_t resident,
-                                         uint32_t iterations, cudaStream_t st) {
-  if (soa) return agg ? launch_atomic<true, true>(d, resident, iterations, st)
-                      : launch_atomic<true, false>(d, resident, iterations, st);
-  return agg ? launch_atomic<false, true>(d, resident, iterations, st)
-             : launch_atomic<false, false>(d, resident, iterations, st);
+                                         uint32_t iterations, bool backwards, cudaStream_t st) {
+  if (soa) return agg ? launch_atomic<true, true>(d, resident, iterations, backwards, st)
+                      : launch_atomic<true, false>(d, resident, iterations, backwards, st);
+  return agg ? launch_atomic<false, true>(d, resident, iterations, backwards, st)
+             : launch_atomic<false, false>(d, resident, iterations, backwards, st);
 }
 
 int FOT_CAT(atomic_occupancy_, FOT_ADAPTER_NS)(bool soa, bool agg, int *per_sm) {
