@@ -1,4 +1,4 @@
-// Batched atomic executor: tiles of kAtomicTile consecutive cells of every
+// Batched atomic executor: tiles of consecutive cells of every
 // mesh and every iteration in one grid-stride launch (iterations need no
 // ordering: the loops never read the dataset they increment).  Compiled with
 // multiply-add contraction, like the single-mesh atomic units (see
@@ -13,26 +13,40 @@
 
 namespace fot {
 
-template <class... Ls> constexpr int max_reg_cap() {
-  int m = 0;
-  ((m = Ls::kRegCap > m ? Ls::kRegCap : m), ...);
+// Resident CTAs per SM: what the loop of the batch that holds most registers
+// runs with on its own.  40 meshes of res_calc and volna, 4,000 to 250,000 cells,
+// an iteration of 2, AOS aggregated / SOA aggregated: 5 CTAs (48 registers) 88.4 /
+// 83.5 us, 4: 92.1 / 85.5, 6: 93.8 / 88.2; 128 and 107 us with 4 and the addresses
+// read through the pointer.
+template <class... Ls> constexpr int batch_min_blocks() {
+  int m = 32;
+  ((m = Ls::kAtomicMinBlocks < m ? Ls::kAtomicMinBlocks : m), ...);
   return m;
 }
 
-template <bool SOA, bool AGG, class... Ls>
-__global__ void __launch_bounds__(256, (65536 / (256 * max_reg_cap<Ls...>())) > 0
-                                           ? 65536 / (256 * max_reg_cap<Ls...>()) : 1)
-    k_batch_atomic(BatchDev B) {
-  const uint32_t warp = threadIdx.x >> 5;
-  for (uint32_t t = blockIdx.x; t < B.total_tiles; t += gridDim.x) {
-    const uint32_t r = t % B.tiles_per_iter;
-    const BatchMesh &m = B.mesh[B.tile_mesh[r]];
-    const uint32_t start = B.tile_block[r];
+// The cells [start, start + cells) of one mesh.  Its addresses are
+// copied first: read through the pointer, they would be read again after
+// every reduction.
+template <class L, bool SOA, bool AGG>
+__device__ __forceinline__ void batch_atomic_tile(const BatchMesh &m, uint32_t start, uint32_t cells) {
+  const LoopData d = m.d;
 #pragma unroll 1
-    for (uint32_t k = 0; k < kAtomicTile / 256; ++k) {
-      const uint32_t base = start + (k * 8u + warp) * 32u;
-      ((m.loop == Ls::kLoop ? (atomic_warp<Ls, SOA, AGG>(m.d, base), 0) : 0), ...);
-    }
+  for (uint32_t k = 0; k < cells; k += 256u)
+    atomic_warp<L, SOA, AGG>(d, start + k + (threadIdx.x & ~31u));
+}
+
+template <bool SOA, bool AGG, class... Ls>
+__global__ void __launch_bounds__(256, batch_min_blocks<Ls...>()) k_batch_atomic(BatchDev B) {
+  griddep_launch_dependents();
+  griddep_wait();
+  for (uint32_t t = blockIdx.x; t < B.total_tiles; t += gridDim.x) {
+    const uint32_t it = t / B.tiles_per_iter, i = t - it * B.tiles_per_iter;
+    // iterations alternate in direction, see AtomicGrid
+    const uint32_t r = (it & 1u) ? B.tiles_per_iter - 1u - i : i;
+    const BatchMesh &m = B.mesh[__ldg(B.tile_mesh + r)];
+    const uint32_t start = __ldg(B.tile_block + r);
+    const int loop = m.loop;
+    ((loop == Ls::kLoop ? (batch_atomic_tile<Ls, SOA, AGG>(m, start, B.tile_cells), 0) : 0), ...);
   }
 }
 

@@ -3,7 +3,7 @@
 //     (iteration, block colour, mesh, block); a tile waits only for its own
 //     mesh's earlier colours, on a per-mesh counter, so meshes of very
 //     different sizes share the GPU without a launch per mesh and colour;
-//   * atomic plans: tiles of 1,024 consecutive cells of one mesh, for every
+//   * atomic plans: tiles of 1,024 (few: 256) consecutive cells of one mesh, for every
 //     mesh and every iteration, in one grid-stride launch (iterations need no
 //     ordering: the loops never read the dataset they increment); that
 //     kernel lives in atomic_batch.cu.
@@ -113,6 +113,7 @@ struct fot_batch {
   int per_sm = 0;
   bool soa = false;
   bool atomic = false;  // atomic plans (else hierarchical)
+  uint32_t tile_cells = kAtomicTile;
   const void *kernel = nullptr;
 };
 
@@ -171,15 +172,21 @@ int fot_batch_create(fot_problem *const *problems, fot_plan *const *plans, uint3
   }
   if (rc == FOT_OK) {
     // tile order: colour-major across meshes, then mesh, then block (atomic
-    // plans: mesh after mesh, kAtomicTile cells per tile)
+    // plans: mesh after mesh, tile_cells cells per tile)
     uint32_t max_col = 0;
     for (auto *pl : B->plans) max_col = std::max(max_col, pl->n_colours);
     std::vector<uint32_t> tm, tb;
     if (B->atomic) {
+      uint64_t tiles = 0;
+      for (auto *p : B->probs) tiles += (p->n_cells + kAtomicTile - 1) / kAtomicTile;
+      int per_sm = 0;
+      if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, B->kernel, (int)B->threads, 0) == cudaSuccess &&
+          tiles < 2ull * per_sm * device_sm_count())
+        B->tile_cells = kAtomicTileSmall;
       for (uint32_t i = 0; i < n; ++i)
-        for (uint32_t c0 = 0; c0 < B->probs[i]->n_cells; c0 += kAtomicTile) {
+        for (uint64_t c0 = 0; c0 < B->probs[i]->n_cells; c0 += B->tile_cells) {
           tm.push_back(i);
-          tb.push_back(c0);
+          tb.push_back((uint32_t)c0);
         }
       max_col = 0;
     }
@@ -237,10 +244,16 @@ int fot_batch_run(fot_batch *B, uint32_t iterations, void *stream) {
   d.tiles_per_iter = B->tiles_per_iter;
   d.total_tiles = (uint32_t)total;
   d.n_mesh = (uint32_t)B->probs.size();
+  d.tile_cells = B->tile_cells;
   d.done = B->done.as<unsigned int>();
   d.ctl = B->ctl.as<Ctl>();
   const uint32_t grid = (uint32_t)std::min<uint64_t>(total, grid_max);
   void *args[] = {&d};
+  if (B->atomic) {
+    Chained c(dim3(grid), dim3(B->threads), B->smem, static_cast<cudaStream_t>(stream));
+    FOT_CUDA(cudaLaunchKernelExC(&c.cfg, B->kernel, args));
+    return FOT_OK;
+  }
   FOT_CUDA(cudaLaunchKernel(B->kernel, dim3(grid), dim3(B->threads), args, B->smem,
                             static_cast<cudaStream_t>(stream)));
   return FOT_OK;

@@ -112,3 +112,17 @@ def test_iterations_of_one_launch(name, layout, iters):
     base, one = md.point_data[0].astype(np.float64), O.serial(md, 1)[0][0].astype(np.float64)
     want = base + iters * (one - base)
     assert rel_err(p.point_weights(0), want) <= (1e-5 if md.loop == mg.VOLNA else 1e-12)
+
+
+@pytest.mark.parametrize("layout", ["aos", "soa"])
+@pytest.mark.parametrize("sizes", [(9, 14, 3), (420, 300, 3)])  # tiles of 256 and of 1,024 cells
+def test_batch_tiles_of_either_size(sizes, layout):
+    side, side2, pairs = sizes
+    mds = [md for i in range(pairs)
+           for md in (mg.res_calc(side, side - i, 5 + i, layout), mg.volna(side2, side2 + i, 5 + i, layout))]
+    probs = [F().Problem.from_mesh(md) for md in mds]
+    b = F().Batch([p.plan(F().EXEC_ATOMIC, 256) for p in probs])
+    b.run(3)
+    b.sync()
+    for md, p in zip(mds, probs):
+        assert rel_err(p.point_weights(0), O.serial(md, 3)[0][0]) <= (1e-5 if md.loop == mg.VOLNA else 1e-12)
