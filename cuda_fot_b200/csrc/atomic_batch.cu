@@ -31,8 +31,11 @@ template <class L, bool SOA, bool AGG>
 __device__ __forceinline__ void batch_atomic_tile(const BatchMesh &m, uint32_t start, uint32_t cells) {
   const LoopData d = m.d;
 #pragma unroll 1
-  for (uint32_t k = 0; k < cells; k += 256u)
-    atomic_warp<L, SOA, AGG>(d, start + k + (threadIdx.x & ~31u));
+  for (uint32_t k = 0; k < cells; k += 256u) {
+    CellMap<L> map;
+    map.load(d, start + k + threadIdx.x);
+    atomic_warp<L, SOA, AGG>(d, start + k + (threadIdx.x & ~31u), map);
+  }
 }
 
 template <bool SOA, bool AGG, class... Ls>

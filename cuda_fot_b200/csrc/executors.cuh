@@ -240,11 +240,21 @@ __device__ __forceinline__ bool sum_runs(uint32_t key, T (&inc)[K]) {
   return (first >> lane) & 1u;
 }
 
+// A cell's rows of the mappings (of a cell past n_cells: unchanged).
+template <class L> struct CellMap {
+  uint32_t p[2][L::kDim] = {};
+  __device__ __forceinline__ void load(const LoopData &d, uint32_t c) {
+    if (c >= d.n_cells) return;
+    load_row<L::kDim>(d.map[0], c, p[0]);
+    if constexpr (L::kHasClass1) load_row<L::kDim>(d.map[1], c, p[1]);
+  }
+};
+
 // Cells [base, base + 32) of one mesh, one per lane of the calling warp
-// (cells past n_cells are masked): compute, optionally sum the runs of lanes
-// with one target point, add with atomics.
+// (cells past n_cells are masked), whose mapping rows are given: compute,
+// optionally sum the runs of lanes with one target point, add with atomics.
 template <class L, bool SOA, bool AGG>
-__device__ __forceinline__ void atomic_warp(const LoopData &d, uint32_t base) {
+__device__ __forceinline__ void atomic_warp(const LoopData &d, uint32_t base, const CellMap<L> &map) {
   using out_t = typename L::out_t;
   constexpr int D = L::kDim, K = L::kOut;
   const uint32_t lane = threadIdx.x & 31u;
@@ -255,14 +265,12 @@ __device__ __forceinline__ void atomic_warp(const LoopData &d, uint32_t base) {
   out_t inc[D][K];
 #pragma unroll
   for (int s = 0; s < D; ++s) {
-    rows.p[0][s] = 0;
-    rows.p[1][s] = 0;
+    rows.p[0][s] = map.p[0][s];
+    rows.p[1][s] = map.p[1][s];
 #pragma unroll
     for (int k = 0; k < K; ++k) inc[s][k] = out_t(0);
   }
   if (valid) {
-    load_row<D>(d.map[0], c, rows.p[0]);
-    if constexpr (L::kHasClass1) load_row<D>(d.map[1], c, rows.p[1]);
     static_for_read<L>([&](auto r) {
       constexpr int R = decltype(r)::value;
       rows.base[R] = static_cast<const typename L::read_t *>(d.point[L::read_set(R)]);
@@ -351,7 +359,8 @@ struct AtomicGrid {
 
 // With L::kAtomicPrefetch, in the SOA form, each warp first prefetches the
 // cells it will take next, so that their mapping rows and direct data come
-// from L2 then.
+// from L2 then; with L::atomic_carry it loads their mapping rows into
+// registers, a memory latency ahead of the rows that they point to.
 template <class L, bool SOA, bool AGG>
 __global__ void __launch_bounds__(256, L::kAtomicMinBlocks) k_atomic(LoopData d, AtomicGrid g) {
   const uint32_t in_tile = threadIdx.x & ~31u, lane = threadIdx.x & 31u;
@@ -361,13 +370,26 @@ __global__ void __launch_bounds__(256, L::kAtomicMinBlocks) k_atomic(LoopData d,
   const bool back = (it + g.flip) & 1u;
   const uint32_t phase = b / g.resident;
   uint32_t t = phase * g.rounds * g.resident + (b - phase * g.resident);
+  constexpr bool kCarry = L::atomic_carry(SOA, AGG);
+  CellMap<L> map;
+  if (kCarry && t < g.tiles) map.load(d, (back ? g.tiles - 1u - t : t) * 256u + in_tile + lane);
   for (uint32_t r = 0; r < g.rounds && t < g.tiles; ++r, t += g.resident) {
+    const uint32_t base = (back ? g.tiles - 1u - t : t) * 256u + in_tile;
+    const uint32_t n = t + g.resident;
+    const uint32_t next = (back ? g.tiles - 1u - n : n) * 256u + in_tile + lane;
+    const bool more = r + 1 < g.rounds && n < g.tiles;
     if constexpr (L::kAtomicPrefetch && SOA) {
-      const uint32_t n = t + g.resident;
-      const uint32_t next = (back ? g.tiles - 1u - n : n) * 256u + in_tile + lane;
-      if (r + 1 < g.rounds && n < g.tiles && next < d.n_cells) prefetch_cell<L>(d, next);
+      if (more && next < d.n_cells) prefetch_cell<L>(d, next);
     }
-    atomic_warp<L, SOA, AGG>(d, (back ? g.tiles - 1u - t : t) * 256u + in_tile);
+    if constexpr (kCarry) {
+      CellMap<L> ahead;
+      if (more) ahead.load(d, next);
+      atomic_warp<L, SOA, AGG>(d, base, map);
+      map = ahead;
+    } else {
+      map.load(d, base + lane);
+      atomic_warp<L, SOA, AGG>(d, base, map);
+    }
   }
 }
 

@@ -97,6 +97,13 @@
 #define FOT_ATOMIC_ABOVE_GETACC 4, 4
 #define FOT_ATOMIC_ROUNDS_GETACC 4
 #endif
+// atomic_carry: whether a warp of the atomic executor loads its next cells'
+// mapping rows while it computes the current ones.  An iteration of 10, warm,
+// without and with: LULESH 96^3 AOS / SOA 41.8 / 37.6 and 40.1 / 37.0 us; res_calc
+// 1000^2 SOA aggregated 27.1 and 25.5 (one iteration with its launch 41.0 and
+// 33.5), AOS 36.3 and 37.0: SOA only; volna 1024^2 AOS 29.8 and 28.7 (43.9 and
+// 42.8), aggregated 30.5 and 32.6: plain only; getacc 1024^2 SOA 34.3 and 35.8,
+// miniAero 128^3 SOA 417 and 417 (its rows are prefetched into L2): off.
 // kDirectRegCap of the adapters below: registers per thread that the direct split
 // write-back kernel is held to; its tiles wait for memory at every step, so
 // that the CTAs an SM holds decide.  Parts of 256, AOS / SOA, by cap: res_calc
@@ -154,6 +161,8 @@ struct Loop {
   static constexpr int kAtomicMinBlocks = FOT_ATOMIC_MINB_RES_CALC;
   // the atomic executor prefetches the next chunk into L2
   static constexpr bool kAtomicPrefetch = FOT_ATOMIC_PREFETCH_RES_CALC;
+  // it loads the next mapping rows ahead
+  __host__ __device__ static constexpr bool atomic_carry(bool soa, bool) { return soa; }
   // phases of its launch: split above so many tiles a CTA (AOS, SOA), this many a phase
   static constexpr uint32_t kAtomicSplitAbove[2] = {FOT_ATOMIC_ABOVE_RES_CALC};
   static constexpr uint32_t kAtomicRounds = FOT_ATOMIC_ROUNDS_RES_CALC;
@@ -201,6 +210,8 @@ struct Loop {
   static constexpr int kAtomicMinBlocks = FOT_ATOMIC_MINB_MINI_AERO;
   // the atomic executor prefetches the next chunk into L2
   static constexpr bool kAtomicPrefetch = FOT_ATOMIC_PREFETCH_MINI_AERO;
+  // it loads the next mapping rows ahead
+  __host__ __device__ static constexpr bool atomic_carry(bool, bool) { return false; }
   // phases of its launch: split above so many tiles a CTA (AOS, SOA), this many a phase
   static constexpr uint32_t kAtomicSplitAbove[2] = {FOT_ATOMIC_ABOVE_MINI_AERO};
   static constexpr uint32_t kAtomicRounds = FOT_ATOMIC_ROUNDS_MINI_AERO;
@@ -258,6 +269,8 @@ struct Loop {
   static constexpr int kAtomicMinBlocks = FOT_ATOMIC_MINB_LULESH;
   // the atomic executor prefetches the next chunk into L2
   static constexpr bool kAtomicPrefetch = FOT_ATOMIC_PREFETCH_LULESH;
+  // it loads the next mapping rows ahead
+  __host__ __device__ static constexpr bool atomic_carry(bool, bool) { return true; }
   // phases of its launch: split above so many tiles a CTA (AOS, SOA), this many a phase
   static constexpr uint32_t kAtomicSplitAbove[2] = {FOT_ATOMIC_ABOVE_LULESH};
   static constexpr uint32_t kAtomicRounds = FOT_ATOMIC_ROUNDS_LULESH;
@@ -313,6 +326,8 @@ struct Loop {
   static constexpr int kAtomicMinBlocks = FOT_ATOMIC_MINB_VOLNA;
   // the atomic executor prefetches the next chunk into L2
   static constexpr bool kAtomicPrefetch = FOT_ATOMIC_PREFETCH_VOLNA;
+  // it loads the next mapping rows ahead
+  __host__ __device__ static constexpr bool atomic_carry(bool, bool agg) { return !agg; }
   // phases of its launch: split above so many tiles a CTA (AOS, SOA), this many a phase
   static constexpr uint32_t kAtomicSplitAbove[2] = {FOT_ATOMIC_ABOVE_VOLNA};
   static constexpr uint32_t kAtomicRounds = FOT_ATOMIC_ROUNDS_VOLNA;
@@ -362,6 +377,8 @@ struct Loop {
   static constexpr int kAtomicMinBlocks = FOT_ATOMIC_MINB_GETACC;
   // the atomic executor prefetches the next chunk into L2
   static constexpr bool kAtomicPrefetch = FOT_ATOMIC_PREFETCH_GETACC;
+  // it loads the next mapping rows ahead
+  __host__ __device__ static constexpr bool atomic_carry(bool, bool) { return false; }
   // phases of its launch: split above so many tiles a CTA (AOS, SOA), this many a phase
   static constexpr uint32_t kAtomicSplitAbove[2] = {FOT_ATOMIC_ABOVE_GETACC};
   static constexpr uint32_t kAtomicRounds = FOT_ATOMIC_ROUNDS_GETACC;
