@@ -105,13 +105,32 @@ struct Direct {
   }
 };
 
-// Read rows straight from global memory (problem layout AOS or SOA).
+// Read rows straight from global memory (problem layout AOS or SOA).  AOS rows
+// of a multiple of 4 doubles are fetched whole, one 32-byte load a sector,
+// where a cell's fit into registers; the user function then reads those:
+// coloured res_calc 1000^2, parts of 256, 48.7 -> 45.9 us.  miniAero's 56 values
+// do not (96^3 AOS 187 us, 257 fetched).
+constexpr int kMostFetched = 16;
 template <class L, bool SOA> struct GlobalRows {
   using T = typename L::read_t;
+  __host__ __device__ static constexpr bool wide(int r) {
+    return !SOA && sizeof(T) == 8 && L::read_dim(r) % 4 == 0;
+  }
+  // values of the wide sets before set r, over all slots
+  __host__ __device__ static constexpr int values_before(int r) {
+    int n = 0;
+    for (int i = 0; i < r; ++i) n += wide(i) ? L::kDim * L::read_dim(i) : 0;
+    return n;
+  }
+  static constexpr bool kFetch = values_before(L::kNumRead) > 0 && values_before(L::kNumRead) <= kMostFetched;
   const T *base[L::kNumRead > 0 ? L::kNumRead : 1];
   unsigned np[L::kNumRead > 0 ? L::kNumRead : 1];
   uint32_t p[2][L::kDim];
+  T fetched[kFetch ? values_before(L::kNumRead) : 1];
+  // takes the datasets; p[][] has been set
+  __device__ __forceinline__ void bind(const LoopData &d);
   template <int R> __device__ __forceinline__ const T *ptr(int s) const {
+    if constexpr (kFetch && wide(R)) return fetched + values_before(R) + s * L::read_dim(R);
     const uint32_t q = p[L::read_class(R)][s];
     const T *r = base[R] + (SOA ? (size_t)q : (size_t)q * L::read_dim(R));
     // AOS rows of a multiple of 16 bytes start 16-byte aligned: the compiler
@@ -145,6 +164,30 @@ __device__ __forceinline__ void static_for_read(F &&f) {
     f(std::integral_constant<int, I>{});
     static_for_read<L, I + 1>(f);
   }
+}
+
+// N values (a multiple of 4 doubles, 32-byte aligned as the rows of datasets are).
+template <int N> __device__ __forceinline__ void load_wide(const double *p, double *v) {
+#pragma unroll
+  for (int k = 0; k < N; k += 4)
+    asm volatile("ld.global.v4.f64 {%0, %1, %2, %3}, [%4];"
+                 : "=d"(v[k]), "=d"(v[k + 1]), "=d"(v[k + 2]), "=d"(v[k + 3])
+                 : "l"(p + k));
+}
+
+template <class L, bool SOA>
+__device__ __forceinline__ void GlobalRows<L, SOA>::bind(const LoopData &d) {
+  static_for_read<L>([&](auto r) {
+    constexpr int R = decltype(r)::value;
+    base[R] = static_cast<const T *>(d.point[L::read_set(R)]);
+    np[R] = d.n_points[L::read_set(R)];
+    if constexpr (kFetch && wide(R)) {
+      constexpr int N = L::read_dim(R);
+#pragma unroll
+      for (int s = 0; s < L::kDim; ++s)
+        load_wide<N>(base[R] + (size_t)p[L::read_class(R)][s] * N, fetched + values_before(R) + s * N);
+    }
+  });
 }
 
 __device__ __forceinline__ size_t out_index(bool soa, uint32_t np0, uint32_t p,
@@ -215,6 +258,58 @@ __device__ __forceinline__ void add_rows_f64(double *__restrict__ out, double *b
   }
 }
 
+// The same for rows of 4, without shared memory: the 4 lanes of a quad transpose
+// their 4x4 values with two exchanges, after which lane q holds component q
+// of the quad's 4 rows.  Neighbouring rows with one key are then neighbouring
+// values of one lane: aggregation (AGG) sums those runs without a shuffle (runs
+// across quads stay separate reductions).  It spares half of the shared-memory
+// passes, and the L1's data path is what bounds loops that gather AOS rows
+// (res_calc 1000^2: 76% busy): with the 32-byte row loads, an iteration of 10
+// after RCM 36.2 -> 33.4 us, aggregated 36.3 -> 28.0.  A loop that gathers none
+// is better off with shared memory's fewer instructions: getacc 1024^2 45.2 us
+// so and 39.2 (aggregated 45.4 and 40.4).
+template <class L> constexpr bool by_quads() {
+  return sizeof(typename L::out_t) == 8 && L::kOut == 4 && L::kNumRead > 0;
+}
+template <bool AGG>
+__device__ __forceinline__ void add_rows4_f64(double *__restrict__ out, uint32_t key, double (&v)[4]) {
+  const uint32_t q = threadIdx.x & 3u;
+  const bool odd = q & 1u, high = q & 2u;
+  // rows 2i, 2i + 1 (lanes q, q ^ 1): components 2i and 2i + 1 change places
+  double a = __shfl_xor_sync(0xFFFFFFFFu, odd ? v[0] : v[1], 1);
+  double b = __shfl_xor_sync(0xFFFFFFFFu, odd ? v[2] : v[3], 1);
+  if (odd) {
+    v[0] = a;
+    v[2] = b;
+  } else {
+    v[1] = a;
+    v[3] = b;
+  }
+  // halves (lanes q, q ^ 2)
+  a = __shfl_xor_sync(0xFFFFFFFFu, high ? v[0] : v[2], 2);
+  b = __shfl_xor_sync(0xFFFFFFFFu, high ? v[1] : v[3], 2);
+  if (high) {
+    v[0] = a;
+    v[1] = b;
+  } else {
+    v[2] = a;
+    v[3] = b;
+  }
+  uint32_t p[4];
+#pragma unroll
+  for (int j = 0; j < 4; ++j) p[j] = __shfl_sync(0xFFFFFFFFu, key, (threadIdx.x & 28u) + j);
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    if constexpr (AGG) {
+      if (j < 3 && p[j] == p[j + 1]) {
+        v[j + 1] += v[j];
+        continue;
+      }
+    }
+    if (p[j] != kNoPoint) atomic_add(out + (size_t)p[j] * 4 + q, v[j]);
+  }
+}
+
 // Warp aggregation: sum the rows of each run of neighbouring lanes with one
 // key into the run's first lane (returns true there).  Orderings sort cells by
 // their points, so that equal keys lie side by side (2 edges, 3 faces of a
@@ -271,17 +366,17 @@ __device__ __forceinline__ void atomic_warp(const LoopData &d, uint32_t base, co
     for (int k = 0; k < K; ++k) inc[s][k] = out_t(0);
   }
   if (valid) {
-    static_for_read<L>([&](auto r) {
-      constexpr int R = decltype(r)::value;
-      rows.base[R] = static_cast<const typename L::read_t *>(d.point[L::read_set(R)]);
-      rows.np[R] = d.n_points[L::read_set(R)];
-    });
+    rows.bind(d);
     Direct dir{d.cell, c, d.n_cells};
     L::cell(rows, dir, inc);
   }
 #pragma unroll
   for (int s = 0; s < D; ++s) {
     const uint32_t key = valid ? rows.p[0][s] : kNoPoint;
+    if constexpr (!SOA && by_quads<L>()) {
+      add_rows4_f64<AGG>(out, key, inc[s]);
+      continue;
+    }
     bool leader = valid;
     if constexpr (AGG) leader = sum_runs<K>(key, inc[s]) && valid;
     if constexpr (!SOA && sizeof(out_t) == 8) {

@@ -159,11 +159,7 @@ __device__ __forceinline__ void tile_compute(const LoopData &d, const HierPlanDe
 #pragma unroll
       for (int s = 0; s < D; ++s) l0[s] = P.lidx[0][(size_t)s * d.n_cells + pos];
       my_col = P.tcol[pos];
-      static_for_read<L>([&](auto r) {
-        constexpr int R = decltype(r)::value;
-        rows.base[R] = static_cast<const read_t *>(d.point[L::read_set(R)]);
-        rows.np[R] = d.n_points[L::read_set(R)];
-      });
+      rows.bind(d);
       Direct dir{d.cell, pos, d.n_cells};
       L::cell(rows, dir, inc);
     }

@@ -149,10 +149,15 @@ template <class L, bool SOA> constexpr bool by_row4() {
 
 // The increments of a tile in shared memory: entry ie = slot * T + cell holds
 // K values, side by side for AOS point data (a point's lanes, or its one
-// 16-byte load, read one row), component by component for SOA.
+// 16-byte load, read one row), component by component for SOA.  Rows of 4
+// doubles swap halves every 4 rows, so that the 16-byte stores of 8 lanes fall
+// into 8 different bank groups (2-way conflicts otherwise: res_calc 1000^2, parts
+// of 256, 51.8 us and 48.7, getacc 1024^2 49.0 and 46.2).
 template <class L, bool SOA, int T>
 __device__ __forceinline__ uint32_t inc_index(uint32_t ie, uint32_t k) {
-  return SOA ? k * (L::kDim * T) + ie : ie * L::kOut + k;
+  if constexpr (SOA) return k * (L::kDim * T) + ie;
+  if constexpr (by_element<L, SOA>() && L::kOut == 4) return ie * 4u + (k ^ ((ie >> 1) & 2u));
+  return ie * L::kOut + k;
 }
 
 template <class L, bool SOA, int T>
@@ -164,7 +169,7 @@ __device__ __forceinline__ void put_increments(typename L::out_t *inc,
     if constexpr (by_element<L, SOA>() && K % 2 == 0) {
 #pragma unroll
       for (int k = 0; k < K; k += 2)
-        *reinterpret_cast<double2 *>(inc + (q * T + t) * K + k) = make_double2(v[q][k], v[q][k + 1]);
+        *reinterpret_cast<double2 *>(inc + inc_index<L, SOA, T>(q * T + t, k)) = make_double2(v[q][k], v[q][k + 1]);
     } else if constexpr (by_row4<L, SOA>()) {
       *reinterpret_cast<float4 *>(inc + (q * T + t) * 4) = make_float4(v[q][0], v[q][1], v[q][2], v[q][3]);
     } else {
@@ -259,7 +264,6 @@ template <class L, int T> constexpr int dsplit_min_blocks() {
 template <class L, bool SOA, int T>
 __global__ void __launch_bounds__(T, dsplit_min_blocks<L, T>()) k_hier_dsplit(LoopData d, HierPlanDev P) {
   using out_t = typename L::out_t;
-  using read_t = typename L::read_t;
   constexpr int D = L::kDim, K = L::kOut;
   extern __shared__ __align__(128) unsigned char smem[];
   __shared__ __align__(8) uint64_t s_full;
@@ -292,11 +296,7 @@ __global__ void __launch_bounds__(T, dsplit_min_blocks<L, T>()) k_hier_dsplit(Lo
     GlobalRows<L, SOA> rows;
     load_row<D>(d.map[0], pos, rows.p[0]);
     if constexpr (L::kHasClass1) load_row<D>(d.map[1], pos, rows.p[1]);
-    static_for_read<L>([&](auto r) {
-      constexpr int R = decltype(r)::value;
-      rows.base[R] = static_cast<const read_t *>(d.point[L::read_set(R)]);
-      rows.np[R] = d.n_points[L::read_set(R)];
-    });
+    rows.bind(d);
     out_t v[D][K];
     Direct dir{d.cell, pos, d.n_cells};
     L::cell(rows, dir, v);

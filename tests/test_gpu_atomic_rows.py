@@ -126,3 +126,17 @@ def test_batch_tiles_of_either_size(sizes, layout):
     b.sync()
     for md, p in zip(mds, probs):
         assert rel_err(p.point_weights(0), O.serial(md, 3)[0][0]) <= (1e-5 if md.loop == mg.VOLNA else 1e-12)
+
+
+@pytest.mark.parametrize("flags", [0, 1])
+@pytest.mark.parametrize("runs", list(RUNS))
+def test_quads_of_rows(runs, flags):
+    """Rows of 4 doubles through the quads of a loop that gathers (res_calc, AOS)."""
+    md = MESHES["res_calc"]("aos")
+    g = np.random.default_rng(9)
+    n, points = md.n_cells, md.n_points[0]
+    run = np.repeat(np.arange(n), np.resize(np.array(RUNS[runs]), n))[:n]
+    rows = np.stack([g.permutation(points)[:2] for _ in range(int(run.max()) + 1)])
+    m = np.ascontiguousarray(rows[run].astype(np.uint32))
+    md.maps = [m, md.maps[1], m.copy(), m.copy()]
+    check(md, flags)
