@@ -30,7 +30,7 @@
 // an iteration of 1000^2 so (169 us as a graph), 173 us fused (165); 300^2 42 and
 // 28.5 us (28.4 and 21.8).  With each kernel started while the one before it
 // drains, and res_calc running against the cell passes' direction (it starts on
-// the cells they left in L2): 163 us (169 in their direction), 300^2 24.8 us.
+// the cells they left in L2): 159 us (165 in their direction), 300^2 21.5 us.
 // Every kernel is compiled without multiply-add
 // contraction, and every sum has a fixed order: boundary edges are added per
 // cell in increasing edge order (one thread per boundary cell), the rms is a
@@ -158,7 +158,6 @@ template <bool UPDATE, bool SAVE, bool ADT, bool RMS>
 __global__ void __launch_bounds__(kThreads, kCellsMinCtas) k_cells(AirfoilDev a, double *partial) {
   __shared__ double smem[kThreads / 32];
   __shared__ bool s_last;
-  griddep_launch_dependents();
   griddep_wait();
   double sum = 0.0;
   const uint32_t stride = gridDim.x * blockDim.x;

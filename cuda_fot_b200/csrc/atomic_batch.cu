@@ -13,15 +13,15 @@
 
 namespace fot {
 
-// Resident CTAs per SM: what the loop of the batch that holds most registers
-// runs with on its own.  40 meshes of res_calc and volna, 4,000 to 250,000 cells,
-// an iteration of 2, AOS aggregated / SOA aggregated: 5 CTAs (48 registers) 88.4 /
-// 83.5 us, 4: 92.1 / 85.5, 6: 93.8 / 88.2; 128 and 107 us with 4 and the addresses
-// read through the pointer.
+// Registers per thread: the most that a loop of the batch asks for in the tile
+// kernels; one CTA an SM more (48 registers for res_calc with volna) spills the
+// addresses: SOA without aggregation, 36 meshes of 2,500 to 70,000 cells, two
+// iterations, 51 us and 58; 40 of 4,000 to 250,000 180 and 190; AOS aggregated 49
+// and 49, 156 and 154.
 template <class... Ls> constexpr int batch_min_blocks() {
-  int m = 32;
-  ((m = Ls::kAtomicMinBlocks < m ? Ls::kAtomicMinBlocks : m), ...);
-  return m;
+  int m = 0;
+  ((m = Ls::kRegCap > m ? Ls::kRegCap : m), ...);
+  return 65536 / (256 * m) > 0 ? 65536 / (256 * m) : 1;
 }
 
 // The cells [start, start + cells) of one mesh.  Its addresses are
@@ -40,7 +40,6 @@ __device__ __forceinline__ void batch_atomic_tile(const BatchMesh &m, uint32_t s
 
 template <bool SOA, bool AGG, class... Ls>
 __global__ void __launch_bounds__(256, batch_min_blocks<Ls...>()) k_batch_atomic(BatchDev B) {
-  griddep_launch_dependents();
   griddep_wait();
   for (uint32_t t = blockIdx.x; t < B.total_tiles; t += gridDim.x) {
     const uint32_t it = t / B.tiles_per_iter, i = t - it * B.tiles_per_iter;

@@ -181,7 +181,7 @@ int fot_batch_create(fot_problem *const *problems, fot_plan *const *plans, uint3
       for (auto *p : B->probs) tiles += (p->n_cells + kAtomicTile - 1) / kAtomicTile;
       int per_sm = 0;
       if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, B->kernel, (int)B->threads, 0) == cudaSuccess &&
-          tiles < 2ull * per_sm * device_sm_count())
+          2 * tiles < 5ull * per_sm * device_sm_count())
         B->tile_cells = kAtomicTileSmall;
       for (uint32_t i = 0; i < n; ++i)
         for (uint64_t c0 = 0; c0 < B->probs[i]->n_cells; c0 += B->tile_cells) {

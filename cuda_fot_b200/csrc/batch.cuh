@@ -28,10 +28,9 @@ struct BatchDev {
 };
 
 // Cells per tile of the atomic batch: the larger one spares look-ups, but a
-// batch that has less than two such tiles for each CTA is over sooner with the
-// smaller (8 meshes of 2,000 to 20,000 cells, one iteration, AOS: 9.2 us and
-// 14.3; 40 of 4,000 to 250,000, 4.5 tiles a CTA: 101 and 100, two iterations 187
-// and 177).
+// batch that has less than 2.5 such tiles for each CTA is over sooner with the
+// smaller: AOS aggregated, one iteration, 1.3 tiles a CTA 16.0 us and 23.8 with
+// the larger, 2.1 26.1 and 28.9, 2.8 38.7 and 35.4, 6.8 98.2 and 88.4.
 constexpr uint32_t kAtomicTile = 1024, kAtomicTileSmall = 256;
 
 // the atomic batch kernel for a set of loop kinds (atomic_batch.cu)

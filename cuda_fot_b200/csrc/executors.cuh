@@ -87,9 +87,9 @@ struct HierPlanDev {
   // per launch: tiles run (0: combine only), the buffer they fill, CTAs
   // combining the other buffer (previous iteration)
   uint32_t tiles_on, put_buf, comb_ctas;
-  // the first launch of a call waits for what precedes it before it reads;
-  // tiles last to first (every other iteration)
-  uint32_t ordered, backwards;
+  // the first launch of a call waits for what precedes it before it reads; the
+  // next launch has tiles too; tiles last to first (every other iteration)
+  uint32_t ordered, more, backwards;
 };
 
 // Direct (cell) data of one cell: SOA with stride n_cells.
@@ -442,8 +442,11 @@ template <class L> __device__ __forceinline__ void prefetch_cell(const LoopData 
 //
 // The grid starts while the one before it on the stream drains and waits for
 // its end (griddep_wait) before it touches memory, which hides the launch:
-// calls of one iteration one after the other, 64x48 res_calc 4.10 us and 3.5 us
-// (the host's rate), volna 300^2 6.2 and 5.3 us.
+// calls of one iteration one after the other, 64x48 res_calc 4.10 us and 3.4 us
+// (the host's rate), volna 300^2 6.2 and 4.4 us, LULESH 30^3 8.3 and 3.9.  It does
+// not let the next grid start before its own CTAs end (which all it could do
+// is wait): with an early griddepcontrol.launch_dependents LULESH 30^3 took 5.9
+// us, res_calc 200x210 4.2 (3.5 without), miniAero 80^3 118 (114).
 struct AtomicGrid {
   uint32_t tiles;     // of one iteration
   uint32_t resident;  // CTAs of a phase
@@ -459,7 +462,6 @@ struct AtomicGrid {
 template <class L, bool SOA, bool AGG>
 __global__ void __launch_bounds__(256, L::kAtomicMinBlocks) k_atomic(LoopData d, AtomicGrid g) {
   const uint32_t in_tile = threadIdx.x & ~31u, lane = threadIdx.x & 31u;
-  griddep_launch_dependents();
   griddep_wait();
   const uint32_t it = blockIdx.x / g.ctas, b = blockIdx.x - it * g.ctas;
   const bool back = (it + g.flip) & 1u;

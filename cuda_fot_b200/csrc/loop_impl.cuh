@@ -105,6 +105,7 @@ int run_hier(const LoopData &d, const HierPlanDev &P, bool soa, uint32_t threads
       Q.put_buf = it & 1u;
       Q.comb_ctas = it > 0 ? comb_ctas : 0u;
       Q.ordered = it == 0;
+      Q.more = it + 1 < iters;
       Q.backwards = (it & 1u) ^ (backwards ? 1u : 0u);
       Chained c(dim3(Q.comb_ctas + (last ? 0u : grid)), dim3(threads), last ? 0 : smem, st);
       FOT_CUDA(cudaLaunchKernelExC(&c.cfg, k, qargs));
