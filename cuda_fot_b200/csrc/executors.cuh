@@ -158,6 +158,14 @@ template <class L> struct SmemRows {
   template <int R> __device__ __forceinline__ unsigned stride() const { return 1u; }
 };
 
+// Direct data whose written value is held back: the cell function's store to
+// cell dataset j goes to *held, for the kernel to store later.
+template <class T> struct HeldDirect : Direct {
+  T *held;
+  __device__ __forceinline__ HeldDirect(const Direct &d, T *h) : Direct(d), held(h) {}
+  template <class U> __device__ __forceinline__ U *wptr(int) const { return held; }
+};
+
 template <class L, int I = 0, class F>
 __device__ __forceinline__ void static_for_read(F &&f) {
   if constexpr (I < L::kNumRead) {

@@ -11,7 +11,8 @@
 //                 mapping class (0: mapping 0; 1: a second, distinct mapping
 //                 such as res_calc's edge->node), dimension, element type
 //   direct sets   cell datasets (SOA), element type, and which are written
-//                 (kWritesCell: the cell function writes a cell dataset)
+//                 (kWritesCell: the cell function writes one value of cell dataset
+//                 kWrittenSet, of type written_t)
 // and a device function cell() that, given row pointers of the read sets for
 // each slot (in global memory or staged in shared memory) and the cell's
 // direct data, produces the signed per-slot increments inc[slot][k] such that
@@ -278,7 +279,9 @@ struct Loop {
   __host__ __device__ static constexpr int read_class(int) { return 0; }
   __host__ __device__ static constexpr int read_dim(int) { return 3; }
   static constexpr int kNumDirect = 2;
-  static constexpr bool kWritesCell = true; // determ (cell dataset 1)
+  static constexpr bool kWritesCell = true; // determ
+  static constexpr int kWrittenSet = 1;
+  using written_t = double;
 
   template <class Rows, class Direct>
   __device__ __forceinline__ static void cell(const Rows &rows, const Direct &dir,
@@ -290,7 +293,7 @@ struct Loop {
     double determ;
     user_func_gpu(f, xyz, dir.template ptr<double>(0), determ,
                   rows.template stride<0>(), dir.stride);
-    *dir.template wptr<double>(1) = determ;
+    *dir.template wptr<written_t>(kWrittenSet) = determ;
 #pragma unroll
     for (int j = 0; j < 8; ++j)
 #pragma unroll
