@@ -308,14 +308,13 @@ def main(argv=None):
 
     md_run = cache.get(chosen.order, chosen.partition, chosen.layout)
     p, plan = T.build(md_run, chosen)
-    # launches of one Plan.run(K) call: the atomic executor launches once per
-    # iteration; the split write-back kernels once per iteration plus one
-    # combine-only launch when blocks share points; the other persistent
-    # hierarchical kernels once per call; the per-colour form once per colour
-    # and iteration
+    # launches of one Plan.run(K) call: the split write-back kernel launches
+    # once per iteration plus one combine-only launch when blocks share points;
+    # the atomic executor and the other persistent hierarchical kernels once
+    # per call; the per-colour form once per colour and iteration
     st0 = plan.stats()
     if chosen.exec == "atomic":
-        launches = args.steps
+        launches = 1
     elif chosen.exec == "hier" and st0["kernel"].startswith("split"):
         launches = args.steps + (1 if st0["shared_points"] else 0)
     elif chosen.exec == "hier":

@@ -197,7 +197,7 @@ static int enqueue_plan(fot_problem *p, fot_plan *plan, uint32_t iterations, boo
   const LoopOps *ops = loop_ops(p->loop);
   const LoopData d = p->loop_data();
   const bool soa = p->layout == FOT_SOA;
-  const int sms = device_sm_count();
+  const int sms = plan->sms;
   if (plan->point_layout != p->layout)
     return fail(FOT_ERR_STATE, "plan is stale: the problem's point layout changed after the plan was built");
   if (plan->desc.exec == FOT_EXEC_ATOMIC) {
@@ -443,6 +443,7 @@ int fot_plan_build(fot_problem *p, const fot_plan_desc *desc, fot_plan **out) {
   plan->prob = p;
   plan->desc = *desc;
   plan->point_layout = p->layout;
+  plan->sms = device_sm_count();
   const LoopOps *ops = loop_ops(p->loop);
   int rc = FOT_OK;
   if (desc->exec == FOT_EXEC_ATOMIC) {

@@ -151,6 +151,7 @@ struct fot_plan {
   size_t smem = 0;
   uint32_t threads = 0;
   int per_sm = 0;
+  int sms = 1; // of the device that the plan was built on
   fot::DevBuf ctl;
   fot::HierPlanDev dev(uint32_t iterations) const;
 };

@@ -41,6 +41,11 @@ _lib = C.CDLL(LIB_PATH)
 _lib.fot_last_error.restype = C.c_char_p
 _lib.fot_version.restype = C.c_char_p
 
+# the call of a time loop: declared, so that its arguments convert without
+# wrapping them one by one
+_fot_run = _lib.fot_run
+_fot_run.argtypes = [C.c_void_p, C.c_void_p, C.c_uint32, C.c_void_p]
+
 u32p = C.POINTER(C.c_uint32)
 
 
@@ -149,7 +154,9 @@ class Plan:
         return arrs
 
     def run(self, iterations: int = 1, stream=None) -> None:
-        _check(_lib.fot_run(self.problem._h, self._h, iterations, _stream_ptr(stream)))
+        rc = _fot_run(self.problem._h, self._h, iterations, None if stream is None else _stream_ptr(stream))
+        if rc != FOT_OK:
+            _check(rc)
 
     def graph(self, iterations: int, stream=None) -> "Graph":
         return Graph(self, iterations, stream)
