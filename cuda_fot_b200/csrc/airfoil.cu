@@ -30,7 +30,8 @@
 // an iteration of 1000^2 so (169 us as a graph), 173 us fused (165); 300^2 42 and
 // 28.5 us (28.4 and 21.8).  With each kernel started while the one before it
 // drains, and res_calc running against the cell passes' direction (it starts on
-// the cells they left in L2): 159 us (165 in their direction), 300^2 21.5 us.
+// the cells they left in L2): 163 us (169 in their direction), 300^2 22.3 us.
+// Asking for a cell's corners before anything is stored: 140 us, 300^2 21.8 us.
 // Every kernel is compiled without multiply-add
 // contraction, and every sum has a fixed order: boundary edges are added per
 // cell in increasing edge order (one thread per boundary cell), the rms is a
@@ -49,16 +50,16 @@ namespace {
 constexpr double kGam = 1.4, kGm1 = 0.4, kEps = 0.05; // gm1 and eps as res_calc_func.hpp
 constexpr uint32_t kThreads = 256;
 #ifndef FOT_AIRFOIL_MAX_CTAS
-#define FOT_AIRFOIL_MAX_CTAS 1184
+#define FOT_AIRFOIL_MAX_CTAS 592
 #endif
 #ifndef FOT_CELLS_MINB
 #define FOT_CELLS_MINB 4
 #endif
-// resident CTAs per SM of a cell pass: the boundary branch needs 62 registers;
-// 5 CTAs spill in it (1000^2 173 us an iteration with 4 and with 5, 176 with 6, 184
-// with 8; AOS 200, 204, 221, 226)
+// resident CTAs per SM of a cell pass (64 registers; 5 spill): 1000^2 an iteration
+// 143 us, 153 with 3, 151 with 5
 constexpr int kCellsMinCtas = FOT_CELLS_MINB;
-// CTAs of a cell pass (grid-stride beyond); the rms sums one partial per CTA
+// CTAs of a cell pass (grid-stride beyond), those the GPU holds at once (1000^2 140
+// us an iteration, 143 with twice as many); the rms sums one partial per CTA
 constexpr uint32_t kMaxUpdateCtas = FOT_AIRFOIL_MAX_CTAS;
 
 struct AirfoilDev {
@@ -83,24 +84,35 @@ __device__ __forceinline__ size_t at(int soa, uint32_t n, uint32_t i, int dim, i
   return soa ? (size_t)k * n + i : (size_t)i * dim + k;
 }
 
-// adt_calc of cell c from its state q.
-__device__ __forceinline__ double cell_adt(const AirfoilDev &a, uint32_t c, const double (&q)[4]) {
-  const uint4 nd = a.cell_nodes[c];
-  const uint32_t node[4] = {nd.x, nd.y, nd.z, nd.w};
+// The corners of a cell with nodes nd.
+struct Corners {
   double px[4], py[4];
+  __device__ __forceinline__ void load(const AirfoilDev &a, const uint4 &nd) {
+    const uint32_t node[4] = {nd.x, nd.y, nd.z, nd.w};
 #pragma unroll
-  for (int j = 0; j < 4; ++j) {
-    px[j] = a.x[at(a.soa, a.n_nodes, node[j], 2, 0)];
-    py[j] = a.x[at(a.soa, a.n_nodes, node[j], 2, 1)];
+    for (int j = 0; j < 4; ++j) {
+      if (a.soa) {
+        px[j] = a.x[node[j]];
+        py[j] = a.x[(size_t)a.n_nodes + node[j]];
+      } else {
+        const double2 xy = *reinterpret_cast<const double2 *>(a.x + 2 * (size_t)node[j]);
+        px[j] = xy.x;
+        py[j] = xy.y;
+      }
+    }
   }
+};
+
+// adt_calc of a cell from its state q.
+__device__ __forceinline__ double cell_adt(const AirfoilDev &a, const Corners &n, const double (&q)[4]) {
   const double ri = 1.0 / q[0];
   const double u = ri * q[1], v = ri * q[2];
   const double snd = sqrt(kGam * kGm1 * (ri * q[3] - 0.5 * (u * u + v * v)));
   double s = 0.0;
 #pragma unroll
   for (int j = 0; j < 4; ++j) {
-    const double dx = px[(j + 1) & 3] - px[j];
-    const double dy = py[(j + 1) & 3] - py[j];
+    const double dx = n.px[(j + 1) & 3] - n.px[j];
+    const double dy = n.py[(j + 1) & 3] - n.py[j];
     s += fabs(u * dy - v * dx) + snd * sqrt(dx * dx + dy * dy);
   }
   return s / a.cfl;
@@ -163,6 +175,13 @@ __global__ void __launch_bounds__(kThreads, kCellsMinCtas) k_cells(AirfoilDev a,
   const uint32_t stride = gridDim.x * blockDim.x;
   for (uint32_t c = blockIdx.x * blockDim.x + threadIdx.x; c < a.n_cells; c += stride) {
     double q[4];
+    // a cell's nodes are asked for first and its corners before anything is
+    // stored: after the stores their two dependent loads would wait for
+    // everything before them (the compiler may not move loads up across
+    // stores)
+    uint4 nodes;
+    Corners corners;
+    if constexpr (ADT) nodes = __ldg(a.cell_nodes + c);
     if constexpr (UPDATE) {
       const double adt = a.adt[c];
       double r[4];
@@ -174,17 +193,22 @@ __global__ void __launch_bounds__(kThreads, kCellsMinCtas) k_cells(AirfoilDev a,
         for (int k = 0; k < 4; ++k) q[k] = a.q[at(a.soa, a.n_cells, c, 4, k)];
         add_boundary(a, a.before[c >> 5] + __popc(word & (bit - 1u)), q, adt, r);
       }
+      double old[4];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) old[k] = a.qold[at(a.soa, a.n_cells, c, 4, k)];
+      if constexpr (ADT) corners.load(a, nodes);
       const double adti = 1.0 / adt;
 #pragma unroll
       for (int k = 0; k < 4; ++k) {
         const size_t o = at(a.soa, a.n_cells, c, 4, k);
         const double del = adti * r[k];
-        q[k] = a.qold[o] - del;
+        q[k] = old[k] - del;
         a.q[o] = q[k];
         a.res[o] = 0.0;
         if constexpr (RMS) sum += del * del;
       }
     } else {
+      if constexpr (ADT) corners.load(a, nodes);
 #pragma unroll
       for (int k = 0; k < 4; ++k) q[k] = a.q[at(a.soa, a.n_cells, c, 4, k)];
     }
@@ -192,7 +216,7 @@ __global__ void __launch_bounds__(kThreads, kCellsMinCtas) k_cells(AirfoilDev a,
 #pragma unroll
       for (int k = 0; k < 4; ++k) a.qold[at(a.soa, a.n_cells, c, 4, k)] = q[k];
     }
-    if constexpr (ADT) a.adt[c] = cell_adt(a, c, q);
+    if constexpr (ADT) a.adt[c] = cell_adt(a, corners, q);
   }
   if constexpr (RMS) {
     const double s = block_sum(sum, smem);
