@@ -116,7 +116,7 @@ def mesh_features(st: dict, stats: dict, layout: str) -> np.ndarray:
 
 
 def plan_features(c: T.Candidate) -> np.ndarray:
-    """8 plan features; the seventh is 1 for the direct (unstaged) form of a
+    """8 plan features; the seventh is 1 for the direct label of a
     hierarchical plan and for an atomic plan without warp aggregation, the
     last 1 for SOA point data."""
     ex = np.zeros(3)

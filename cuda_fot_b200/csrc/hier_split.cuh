@@ -318,6 +318,7 @@ __global__ void __launch_bounds__(T, dsplit_min_blocks<L, T>()) k_hier_dsplit(Lo
   __syncthreads();
   if (!mbar_wait(&s_full, 0)) {
     if (tid == 0) atomicOr(&P.ctl->error, kErrWaitLimit);
+    griddep_wait();
     return;
   }
   griddep_wait();  // the previous iteration's writes are visible

@@ -7,7 +7,7 @@ Builds the mesh and the plan, then calls Plan.run(1) `--launches` times, so a
 profiler can skip the first launches (-s) and capture one to three (-c) of the
 same kernel.  With --airfoil (res_calc only) it runs that many Airfoil
 solver iterations around the plan instead (fot_airfoil_run: the cell passes
-k_cells, k_bres_calc, k_rms and the plan's res_calc kernel).  Plan labels are those of cuda_fot_b200.tune.Candidate.label():
+k_cells and the plan's res_calc kernel).  Plan labels are those of cuda_fot_b200.tune.Candidate.label():
 `order[+partN]/exec[d][-plain]/block[@soa]`, e.g. `gps/hier/128`,
 `gps+part256/hierd/256`, `as-is/atomic-plain/256@soa`.  Sizes: res_calc/volna/getacc take --n as the grid edge
 (n x n), mini_aero/lulesh as the hex edge (n^3).

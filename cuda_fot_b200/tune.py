@@ -7,9 +7,9 @@ A candidate is (ordering, partition size, executor, block size, layout):
 * partition -- 0, or the part size of fot_partition followed by
   fot_reorder_to_partition and fot_renumber_points (the reference's
   partition -> reorderToPartition -> renumberPoints sequence);
-* executor  -- "atomic", "hier" (persistent; split write-back kernel,
-  staged or -- with direct -- gathering rows straight from HBM/L2) or
-  "hier_launch";
+* executor  -- "atomic", "hier" (persistent; the split write-back kernel, with
+  and without direct) or "hier_launch" (read rows staged or -- with direct --
+  gathered straight from HBM/L2);
 * block     -- cells per block (hierarchical) / threads per CTA (atomic);
 * layout    -- "aos" or "soa" point data (the reference's Problem<SOA>).
 
@@ -55,8 +55,8 @@ class Candidate:
 def plan_candidates(order: Optional[str], part: int) -> List[Candidate]:
     """The plans of one (ordering, partition): for both point layouts, the
     atomic executor with and without warp aggregation and the hierarchical
-    executor's staged and direct split write-back kernels (blocks of 128, 256,
-    512 and 128, 256 cells; on a partition, blocks of the part size)."""
+    executor's split write-back kernel under both of its labels (blocks of 128,
+    256, 512 and 128, 256 cells; on a partition, blocks of the part size)."""
     out = []
     for lay in ("aos", "soa"):
         out.append(Candidate(order, part, "atomic", 256, layout=lay))
