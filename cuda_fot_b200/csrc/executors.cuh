@@ -437,8 +437,10 @@ template <class L> __device__ __forceinline__ void prefetch_cell(const LoopData 
 // phase against one phase for all: miniAero SOA 128^3 421 us (R = 4) and 585,
 // 120^3 342 and 352, but 96^3 177 and 172 (23 rounds in all: not split);
 // getacc 1024^2 43.4 and 45.1 (AOS), 1500x1600 SOA 88.7 and 101.1; volna 1024^2
-// 39.8 and 40.9 (R = 8); res_calc 2000x1900 SOA 133 and 130, LULESH 96^3 46.2
-// and 46.2 (never split), miniAero AOS 128^3 489 and 447 (never split).
+// 39.8 and 40.9 (R = 8); res_calc SOA without aggregation, fresh data, 1000^2
+// 37.3 and 38.9, 1200^2 51.5 and 55.1, 2000^2 133 and 149 (R = 6), aggregated 1200^2
+// 43.7 and 41.6, AOS 1000^2 34.0 and 33.3 (neither split); LULESH 96^3 44.2 and
+// 44.1, miniAero AOS 128^3 489 and 447 (never split).
 //
 // The iterations of a call are one launch as well (no iteration reads what
 // another writes), each running through the mesh in the direction opposite to

@@ -31,9 +31,8 @@ int launch_atomic(const LoopData &d, uint32_t resident, uint32_t iterations, boo
   g.tiles = (d.n_cells + 255u) / 256u;
   g.resident = std::max(1u, std::min(g.tiles, resident));
   const uint32_t all = (g.tiles + g.resident - 1) / g.resident;
-  const uint32_t phases = LA::kAtomicSplitAbove[SOA] && all > LA::kAtomicSplitAbove[SOA]
-                              ? (all + LA::kAtomicRounds - 1) / LA::kAtomicRounds
-                              : 1;
+  constexpr uint32_t above = LA::kAtomicSplitAbove[2 * SOA + AGG];
+  const uint32_t phases = above && all > above ? (all + LA::kAtomicRounds - 1) / LA::kAtomicRounds : 1;
   g.rounds = (all + phases - 1) / phases;
   g.ctas = phases * g.resident;
   const uint32_t most = std::max(1u, (1u << 30) / g.ctas);

@@ -76,26 +76,27 @@
 #define FOT_ATOMIC_MINB_GETACC 2
 #endif
 // Phases of the atomic executor's launch (AtomicGrid): split when a CTA would
-// take more than ABOVE tiles (AOS, SOA; 0: never), into phases of ROUNDS tiles
-// a CTA; the measurements are at AtomicGrid.
+// take more than ABOVE tiles (AOS plain, AOS aggregated, SOA plain, SOA
+// aggregated; 0: never), into phases of ROUNDS tiles a CTA; the measurements are
+// at AtomicGrid.
 #ifndef FOT_ATOMIC_ABOVE_RES_CALC
-#define FOT_ATOMIC_ABOVE_RES_CALC 0, 0
-#define FOT_ATOMIC_ROUNDS_RES_CALC 1
+#define FOT_ATOMIC_ABOVE_RES_CALC 0, 0, 6, 0
+#define FOT_ATOMIC_ROUNDS_RES_CALC 6
 #endif
 #ifndef FOT_ATOMIC_ABOVE_MINI_AERO
-#define FOT_ATOMIC_ABOVE_MINI_AERO 0, 24
+#define FOT_ATOMIC_ABOVE_MINI_AERO 0, 0, 24, 24
 #define FOT_ATOMIC_ROUNDS_MINI_AERO 4
 #endif
 #ifndef FOT_ATOMIC_ABOVE_LULESH
-#define FOT_ATOMIC_ABOVE_LULESH 0, 0
+#define FOT_ATOMIC_ABOVE_LULESH 0, 0, 0, 0
 #define FOT_ATOMIC_ROUNDS_LULESH 1
 #endif
 #ifndef FOT_ATOMIC_ABOVE_VOLNA
-#define FOT_ATOMIC_ABOVE_VOLNA 8, 8
+#define FOT_ATOMIC_ABOVE_VOLNA 8, 8, 8, 8
 #define FOT_ATOMIC_ROUNDS_VOLNA 8
 #endif
 #ifndef FOT_ATOMIC_ABOVE_GETACC
-#define FOT_ATOMIC_ABOVE_GETACC 4, 4
+#define FOT_ATOMIC_ABOVE_GETACC 4, 4, 4, 4
 #define FOT_ATOMIC_ROUNDS_GETACC 4
 #endif
 // atomic_carry: whether a warp of the atomic executor loads its next cells'
@@ -164,8 +165,9 @@ struct Loop {
   static constexpr bool kAtomicPrefetch = FOT_ATOMIC_PREFETCH_RES_CALC;
   // it loads the next mapping rows ahead
   __host__ __device__ static constexpr bool atomic_carry(bool soa, bool) { return soa; }
-  // phases of its launch: split above so many tiles a CTA (AOS, SOA), this many a phase
-  static constexpr uint32_t kAtomicSplitAbove[2] = {FOT_ATOMIC_ABOVE_RES_CALC};
+  // phases of its launch: split above so many tiles a CTA ([2 * SOA + aggregated]),
+  // this many a phase
+  static constexpr uint32_t kAtomicSplitAbove[4] = {FOT_ATOMIC_ABOVE_RES_CALC};
   static constexpr uint32_t kAtomicRounds = FOT_ATOMIC_ROUNDS_RES_CALC;
   // read set r: x (set 1, class 1, dim 2), q (set 2, class 0, dim 4), adt (set 3, class 0, dim 1)
   __host__ __device__ static constexpr int read_set(int r) { return r + 1; }
@@ -213,8 +215,9 @@ struct Loop {
   static constexpr bool kAtomicPrefetch = FOT_ATOMIC_PREFETCH_MINI_AERO;
   // it loads the next mapping rows ahead
   __host__ __device__ static constexpr bool atomic_carry(bool, bool) { return false; }
-  // phases of its launch: split above so many tiles a CTA (AOS, SOA), this many a phase
-  static constexpr uint32_t kAtomicSplitAbove[2] = {FOT_ATOMIC_ABOVE_MINI_AERO};
+  // phases of its launch: split above so many tiles a CTA ([2 * SOA + aggregated]),
+  // this many a phase
+  static constexpr uint32_t kAtomicSplitAbove[4] = {FOT_ATOMIC_ABOVE_MINI_AERO};
   static constexpr uint32_t kAtomicRounds = FOT_ATOMIC_ROUNDS_MINI_AERO;
   __host__ __device__ static constexpr int read_set(int) { return 1; }
   __host__ __device__ static constexpr int read_class(int) { return 0; }
@@ -272,8 +275,9 @@ struct Loop {
   static constexpr bool kAtomicPrefetch = FOT_ATOMIC_PREFETCH_LULESH;
   // it loads the next mapping rows ahead
   __host__ __device__ static constexpr bool atomic_carry(bool, bool) { return true; }
-  // phases of its launch: split above so many tiles a CTA (AOS, SOA), this many a phase
-  static constexpr uint32_t kAtomicSplitAbove[2] = {FOT_ATOMIC_ABOVE_LULESH};
+  // phases of its launch: split above so many tiles a CTA ([2 * SOA + aggregated]),
+  // this many a phase
+  static constexpr uint32_t kAtomicSplitAbove[4] = {FOT_ATOMIC_ABOVE_LULESH};
   static constexpr uint32_t kAtomicRounds = FOT_ATOMIC_ROUNDS_LULESH;
   __host__ __device__ static constexpr int read_set(int) { return 1; }
   __host__ __device__ static constexpr int read_class(int) { return 0; }
@@ -331,8 +335,9 @@ struct Loop {
   static constexpr bool kAtomicPrefetch = FOT_ATOMIC_PREFETCH_VOLNA;
   // it loads the next mapping rows ahead
   __host__ __device__ static constexpr bool atomic_carry(bool, bool agg) { return !agg; }
-  // phases of its launch: split above so many tiles a CTA (AOS, SOA), this many a phase
-  static constexpr uint32_t kAtomicSplitAbove[2] = {FOT_ATOMIC_ABOVE_VOLNA};
+  // phases of its launch: split above so many tiles a CTA ([2 * SOA + aggregated]),
+  // this many a phase
+  static constexpr uint32_t kAtomicSplitAbove[4] = {FOT_ATOMIC_ABOVE_VOLNA};
   static constexpr uint32_t kAtomicRounds = FOT_ATOMIC_ROUNDS_VOLNA;
   __host__ __device__ static constexpr int read_set(int) { return 1; }
   __host__ __device__ static constexpr int read_class(int) { return 0; }
@@ -382,8 +387,9 @@ struct Loop {
   static constexpr bool kAtomicPrefetch = FOT_ATOMIC_PREFETCH_GETACC;
   // it loads the next mapping rows ahead
   __host__ __device__ static constexpr bool atomic_carry(bool, bool) { return false; }
-  // phases of its launch: split above so many tiles a CTA (AOS, SOA), this many a phase
-  static constexpr uint32_t kAtomicSplitAbove[2] = {FOT_ATOMIC_ABOVE_GETACC};
+  // phases of its launch: split above so many tiles a CTA ([2 * SOA + aggregated]),
+  // this many a phase
+  static constexpr uint32_t kAtomicSplitAbove[4] = {FOT_ATOMIC_ABOVE_GETACC};
   static constexpr uint32_t kAtomicRounds = FOT_ATOMIC_ROUNDS_GETACC;
   __host__ __device__ static constexpr int read_set(int) { return 0; }
   __host__ __device__ static constexpr int read_class(int) { return 0; }

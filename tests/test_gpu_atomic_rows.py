@@ -92,6 +92,7 @@ def test_contracted_face_flux(layout):
 # tiles than the GPU holds CTAs, a few rounds, and more rounds than one phase
 SIZES = {"getacc_small": lambda lay: mg.getacc(33, 21, 5, lay), "getacc_phases": lambda lay: mg.getacc(1100, 905, 5, lay),
          "volna_phases": lambda lay: mg.volna(1003, 997, 5, lay), "res_calc": lambda lay: mg.res_calc(301, 299, 5, lay),
+         "res_calc_phases": lambda lay: mg.res_calc(811, 803, 5, lay),
          "mini_aero_phases": lambda lay: mg.mini_aero(103, 5, lay, permute=False),
          "lulesh": lambda lay: mg.lulesh(31, 5, lay)}
 
