@@ -87,8 +87,9 @@ struct HierPlanDev {
   // per launch: tiles run (0: combine only), the buffer they fill, CTAs
   // combining the other buffer (previous iteration)
   uint32_t tiles_on, put_buf, comb_ctas;
-  // the first launch of a call waits for what precedes it before it reads; the
-  // next launch has tiles too; tiles last to first (every other iteration)
+  // the first launch of a call waits for what precedes it before it reads and
+  // before it lets the next start; the next launch has tiles too; tiles last to
+  // first (every other iteration)
   uint32_t ordered, more, backwards;
 };
 

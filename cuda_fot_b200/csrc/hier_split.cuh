@@ -18,10 +18,11 @@
 //     disjoint, so the combine never races with the tiles.
 // Block colours therefore fix the summation order but never stall a tile.
 // One launch runs ONE iteration; consecutive launches are chained with
-// programmatic dependent launch: every CTA lets the next grid start at once,
-// and the next grid's tiles gather and compute (they only read datasets the
-// loop never writes) before they wait (griddepcontrol.wait) for this grid to
-// complete and only then write.  What a cell function writes to cell data is
+// programmatic dependent launch: every CTA lets the next grid start at once
+// (in a call's first grid: once what precedes the call is complete), and the
+// next grid's tiles gather and compute (they only read datasets the loop never
+// writes) before they wait (griddepcontrol.wait) for this grid to complete and
+// only then write.  What a cell function writes to cell data is
 // held in a register until then (LULESH 45^3, 2 iterations 24.2 us waiting before
 // it computes, 22.8 so; 10 iterations 103 and 88; 30^3 68 and 56).
 //
@@ -276,13 +277,18 @@ __global__ void __launch_bounds__(T, dsplit_min_blocks<L, T>()) k_hier_dsplit(Lo
   __shared__ __align__(8) uint64_t s_full;
   out_t *const inc = reinterpret_cast<out_t *>(smem + P.inc_off);
   const uint32_t tid = threadIdx.x;
+  // The first grid of a call waits before it lets the next one start: what
+  // precedes the call may write what tiles read, and the next grid's tiles
+  // read before their own wait.  Triggering first, they could start while that
+  // work still runs (a kernel that lets its dependents start early, or whose
+  // writes are not flushed yet) and gather what it has not written.
+  if (P.ordered) griddep_wait();
   // Where the next grid has tiles that can gather and compute meanwhile, let it
   // start; one that can only wait (the flush) takes longer when it starts
   // early: res_calc 200x210, one iteration, 9.2 us and 6.5, LULESH 30^3 13.1 and
   // 9.4; res_calc 1000^2, 10 iterations, 450 us with the early start and 465
   // without.
   if (P.more) griddep_launch_dependents();
-  if (P.ordered) griddep_wait();  // what precedes a call may write what its tiles read
   const uint32_t n_tiles = P.tiles_on ? P.n_blocks : 0u;
   if (blockIdx.x >= n_tiles) {
     // the combine CTAs come last, so that the tiles are scheduled first

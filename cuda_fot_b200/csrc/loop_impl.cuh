@@ -88,8 +88,9 @@ int run_hier(const LoopData &d, const HierPlanDev &P, bool soa, uint32_t threads
     // combine-only launch flushes the final iteration's buffer.  Programmatic
     // dependent launch lets each grid start while the one before it drains:
     // from the second launch on it gathers and computes before it waits (the
-    // kernel waits before it writes), in the first it waits at once, because
-    // whatever precedes a call may write the datasets it reads.  Iterations
+    // kernel waits before it writes); the first waits before it reads and
+    // before it lets the second start, because whatever precedes a call may
+    // write the datasets that both read.  Iterations
     // alternate in direction, so that each starts on what the one before it
     // left in L2 (parts of 256, 10 iterations, warm: res_calc 1000^2 AOS 54.7 us
     // an iteration in one direction, 51.6 alternating; getacc 1024^2 52.6 and
