@@ -276,6 +276,15 @@ int upload(DevBuf &b, const void *host, size_t bytes) {
   return FOT_OK;
 }
 
+// Copies from pageable memory and memsets may still be under way on the default
+// stream when their calls return.  A run on a non-blocking stream does not wait
+// for that stream, and a count of arrived CTAs cleared in the middle of a pass
+// would never come to its end again: nothing is handed out before they are done.
+int finish_uploads() {
+  FOT_CUDA(cudaStreamSynchronize(nullptr));
+  return FOT_OK;
+}
+
 // Rebuild the device maps for the problem's current numbering.
 int airfoil_renumber(fot_airfoil *a) {
   fot_problem *p = a->prob;
@@ -314,6 +323,7 @@ int airfoil_renumber(fot_airfoil *a) {
   FOT_TRY(upload(a->d_bcell_off, boff.data(), boff.size() * sizeof(uint32_t)));
   FOT_TRY(upload(a->d_bedge_nodes, bnodes.data(), bnodes.size() * sizeof(uint32_t)));
   FOT_TRY(upload(a->d_bedge_bound, bb.data(), bb.size() * sizeof(int32_t)));
+  FOT_TRY(finish_uploads());
   a->version = p->version;
   return FOT_OK;
 }
@@ -360,6 +370,7 @@ int fot_airfoil_create(fot_problem *p, const fot_airfoil_desc *desc, fot_airfoil
   if (rc == FOT_OK && (cudaMemset(a->rms.ptr, 0, sizeof(double)) != cudaSuccess ||
                        cudaMemset(a->arrived.ptr, 0, sizeof(unsigned int)) != cudaSuccess))
     rc = fail(FOT_ERR_CUDA, "cudaMemset failed");
+  if (rc == FOT_OK) rc = finish_uploads();
   if (rc != FOT_OK) {
     delete a;
     return rc;
