@@ -208,6 +208,10 @@ int fot_batch_create(fot_problem *const *problems, fot_plan *const *plans, uint3
     if (rc == FOT_OK && (cudaMemset(B->done.ptr, 0, (size_t)n * 4) != cudaSuccess ||
                          cudaMemset(B->ctl.ptr, 0, sizeof(Ctl)) != cudaSuccess))
       rc = fail(FOT_ERR_CUDA, "memset failed");
+    // a run on a non-blocking stream does not wait for the default one, on which
+    // the copies and memsets above may still be under way
+    if (rc == FOT_OK && cudaStreamSynchronize(nullptr) != cudaSuccess)
+      rc = fail(FOT_ERR_CUDA, "batch creation: the default stream failed");
   }
   if (rc == FOT_OK) {
     const cudaError_t e1 = cudaFuncSetAttribute(B->kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,

@@ -7,7 +7,7 @@ import pytest
 
 from cuda_fot_b200 import meshgen as mg
 from oracle import oracle_py as O
-from tests.helpers import bitwise_equal
+from tests.helpers import bitwise_equal, rel_err
 
 pytestmark = pytest.mark.gpu
 
@@ -62,3 +62,24 @@ def test_airfoil_rms_counts_from_zero():
     af.run(plan, 1, st, rms=False)
     ref, rms = O.airfoil(md, ex, 3, plan.export())
     assert abs(af.rms(st) - rms) <= 1e-12 * rms
+
+
+@pytest.mark.parametrize("kernel", ["atomic", "coloured"])
+def test_batch_starts_from_a_clear_queue(kernel):
+    import torch
+    mds = [mg.res_calc(24, 20, 5), mg.res_calc(17, 9, 6)]
+    probs = [F().Problem.from_mesh(md) for md in mds]
+    plans = [p.plan(F().EXEC_HIER, 128) if kernel == "coloured" else p.plan(F().EXEC_ATOMIC, 256) for p in probs]
+    st = torch.cuda.Stream()
+    with BusyDefaultStream():
+        b = F().Batch(plans)
+        b.run(2, st)
+        st.synchronize()
+    torch.cuda.synchronize()
+    b.run(1, st)
+    b.sync(st)
+    for md, p, plan in zip(mds, probs, plans):
+        if kernel == "coloured":
+            assert bitwise_equal(p.point_weights(0), O.replay_hier(md, plan.export(), 3)[0][0])
+        else:
+            assert rel_err(p.point_weights(0), O.serial(md, 3)[0][0]) <= 1e-12
