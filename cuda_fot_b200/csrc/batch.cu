@@ -114,6 +114,7 @@ struct fot_batch {
   bool soa = false;
   bool atomic = false;  // atomic plans (else hierarchical)
   uint32_t tile_cells = kAtomicTile;
+  uint64_t counted_tiles = 0;  // tiles that the limit of a call's iterations counts
   const void *kernel = nullptr;
 };
 
@@ -177,7 +178,7 @@ int fot_batch_create(fot_problem *const *problems, fot_plan *const *plans, uint3
     for (auto *pl : B->plans) max_col = std::max(max_col, pl->n_colours);
     std::vector<uint32_t> tm, tb;
     if (B->atomic) {
-      uint64_t tiles = 0;
+      uint64_t &tiles = B->counted_tiles;
       for (auto *p : B->probs) tiles += (p->n_cells + kAtomicTile - 1) / kAtomicTile;
       int per_sm = 0;
       if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, B->kernel, (int)B->threads, 0) == cudaSuccess &&
@@ -200,6 +201,7 @@ int fot_batch_create(fot_problem *const *problems, fot_plan *const *plans, uint3
         }
       }
     B->tiles_per_iter = (uint32_t)tm.size();
+    if (!B->atomic) B->counted_tiles = B->tiles_per_iter;
     rc = upload(B->tile_mesh, tm);
     if (rc == FOT_OK) rc = upload(B->tile_block, tb);
     if (rc == FOT_OK) rc = upload(B->mesh, meshes);
@@ -238,28 +240,38 @@ int fot_batch_run(fot_batch *B, uint32_t iterations, void *stream) {
     if (B->probs[i]->version != B->versions[i] ||
         (!B->atomic && B->plans[i]->version != B->versions[i]))
       return fail(FOT_ERR_STATE, "batch entry %zu changed since the batch was created", i);
-  const uint64_t total = (uint64_t)iterations * B->tiles_per_iter;
+  // the limit counts kAtomicTile cells a tile whatever tiles the batch runs by
   const uint32_t grid_max = (uint32_t)(B->per_sm * device_sm_count());
-  if (total + grid_max >= 0xFFFFFFFFull) return fail(FOT_ERR_LIMIT, "too many tiles in one launch");
+  if ((uint64_t)iterations * B->counted_tiles + grid_max >= 0xFFFFFFFFull)
+    return fail(FOT_ERR_LIMIT, "too many tiles in one launch");
   BatchDev d{};
   d.mesh = B->mesh.as<BatchMesh>();
   d.tile_mesh = B->tile_mesh.as<uint32_t>();
   d.tile_block = B->tile_block.as<uint32_t>();
   d.tiles_per_iter = B->tiles_per_iter;
-  d.total_tiles = (uint32_t)total;
   d.n_mesh = (uint32_t)B->probs.size();
   d.tile_cells = B->tile_cells;
   d.done = B->done.as<unsigned int>();
   d.ctl = B->ctl.as<Ctl>();
-  const uint32_t grid = (uint32_t)std::min<uint64_t>(total, grid_max);
   void *args[] = {&d};
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
   if (B->atomic) {
-    Chained c(dim3(grid), dim3(B->threads), B->smem, static_cast<cudaStream_t>(stream));
-    FOT_CUDA(cudaLaunchKernelExC(&c.cfg, B->kernel, args));
+    // a launch counts its tiles in 32 bits: iterations that fit into a call by
+    // the larger tiles but not by the smaller take several launches, of an even
+    // number of iterations each so that directions go on alternating
+    const uint32_t most = (uint32_t)((0xFFFFFFFEull - grid_max) / B->tiles_per_iter);
+    while (iterations) {
+      const uint32_t now = iterations <= most ? iterations : most & ~1u;
+      d.total_tiles = now * B->tiles_per_iter;
+      Chained c(dim3(std::min(d.total_tiles, grid_max)), dim3(B->threads), B->smem, st);
+      FOT_CUDA(cudaLaunchKernelExC(&c.cfg, B->kernel, args));
+      iterations -= now;
+    }
     return FOT_OK;
   }
-  FOT_CUDA(cudaLaunchKernel(B->kernel, dim3(grid), dim3(B->threads), args, B->smem,
-                            static_cast<cudaStream_t>(stream)));
+  d.total_tiles = iterations * B->tiles_per_iter;
+  FOT_CUDA(cudaLaunchKernel(B->kernel, dim3(std::min(d.total_tiles, grid_max)), dim3(B->threads), args,
+                            B->smem, st));
   return FOT_OK;
 }
 
