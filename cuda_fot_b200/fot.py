@@ -15,6 +15,7 @@ module raises if the library has not been built
 from __future__ import annotations
 
 import ctypes as C
+import operator
 import os
 from typing import List, Optional
 
@@ -41,10 +42,10 @@ _lib = C.CDLL(LIB_PATH)
 _lib.fot_last_error.restype = C.c_char_p
 _lib.fot_version.restype = C.c_char_p
 
-# the call of a time loop: declared, so that its arguments convert without
-# wrapping them one by one
+# the call of a time loop, undeclared: handles are c_void_p already, None is the
+# null stream, and an integer converts as it is unless it is beyond 64 bits,
+# which is refused (a declared uint32 takes its low bits: 2**64 would be 0)
 _fot_run = _lib.fot_run
-_fot_run.argtypes = [C.c_void_p, C.c_void_p, C.c_uint32, C.c_void_p]
 
 u32p = C.POINTER(C.c_uint32)
 
@@ -154,6 +155,8 @@ class Plan:
         return arrs
 
     def run(self, iterations: int = 1, stream=None) -> None:
+        if iterations.__class__ is not int and not isinstance(iterations, C.c_uint32):
+            iterations = operator.index(iterations)  # numpy's integers; raises for what is none
         rc = _fot_run(self.problem._h, self._h, iterations, None if stream is None else _stream_ptr(stream))
         if rc != FOT_OK:
             _check(rc)
