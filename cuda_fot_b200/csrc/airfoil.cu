@@ -26,12 +26,13 @@
 // between iterations + save_soln), whose last CTA sums the rms: an iteration
 // is two res_calc runs and two cell passes.  bres_calc (4 edges of a cell at
 // most, here) and the rms as launches of their own were 3 of 7 launches an
-// iteration, each a few us of start and drain for next to no work: 185 us
-// an iteration of 1000^2 so (169 us as a graph), 173 us fused (165); 300^2 42 and
-// 28.5 us (28.4 and 21.8).  With each kernel started while the one before it
-// drains, and res_calc running against the cell passes' direction (it starts on
-// the cells they left in L2): 163 us (169 in their direction), 300^2 22.3 us.
-// Asking for a cell's corners before anything is stored: 140 us, 300^2 21.8 us.
+// iteration, each a few us of start and drain for next to no work: an
+// iteration of 1000^2 was 185 us so (169 us as a graph) and 173 us (165) once
+// fused; it is 141 us (141) now, 300^2 22.7 us.  Of that: each kernel started
+// while the one before it drains (152 us without, 300^2 31.9), res_calc running
+// against the cell passes' direction (it starts on the cells they left in L2:
+// 150 us in their direction), a cell's corners asked for before anything is
+// stored (163 us before that step).
 // Every kernel is compiled without multiply-add
 // contraction, and every sum has a fixed order: boundary edges are added per
 // cell in increasing edge order (one thread per boundary cell), the rms is a
@@ -56,10 +57,11 @@ constexpr uint32_t kThreads = 256;
 #define FOT_CELLS_MINB 4
 #endif
 // resident CTAs per SM of a cell pass (64 registers; 5 spill): 1000^2 an iteration
-// 143 us, 153 with 3, 151 with 5
+// 141 us, 148 with 3, 147 with 5
 constexpr int kCellsMinCtas = FOT_CELLS_MINB;
-// CTAs of a cell pass (grid-stride beyond), those the GPU holds at once (1000^2 140
-// us an iteration, 143 with twice as many); the rms sums one partial per CTA
+// CTAs of a cell pass (grid-stride beyond): those a B200 holds at once, 148 SMs x 4
+// (1000^2 141 us an iteration, 144 with twice as many).  Only speed and the order
+// of the rms's sum follow it, which is one partial per CTA.
 constexpr uint32_t kMaxUpdateCtas = FOT_AIRFOIL_MAX_CTAS;
 
 struct AirfoilDev {

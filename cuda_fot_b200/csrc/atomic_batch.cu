@@ -15,9 +15,9 @@ namespace fot {
 
 // Registers per thread: the most that a loop of the batch asks for in the tile
 // kernels; one CTA an SM more (48 registers for res_calc with volna) spills the
-// addresses: SOA without aggregation, 36 meshes of 2,500 to 70,000 cells, two
-// iterations, 51 us and 58; 40 of 4,000 to 250,000 180 and 190; AOS aggregated 49
-// and 49, 156 and 154.
+// addresses.  An iteration of two, so and with one more: SOA without aggregation,
+// 36 meshes of 2,500 to 70,000 cells 27.3 us and 34.1, 40 of 4,000 to 250,000 94.5
+// and 98.9; AOS aggregated 25.1 and 26.8, 83.3 and 80.0 (98.7 and 87.8 alone).
 template <class... Ls> constexpr int batch_min_blocks() {
   int m = 0;
   ((m = Ls::kRegCap > m ? Ls::kRegCap : m), ...);

@@ -3,10 +3,10 @@
 //     (iteration, block colour, mesh, block); a tile waits only for its own
 //     mesh's earlier colours, on a per-mesh counter, so meshes of very
 //     different sizes share the GPU without a launch per mesh and colour;
-//   * atomic plans: tiles of 1,024 (few: 256) consecutive cells of one mesh, for every
-//     mesh and every iteration, in one grid-stride launch (iterations need no
-//     ordering: the loops never read the dataset they increment); that
-//     kernel lives in atomic_batch.cu.
+//   * atomic plans: tiles of 1,024 (small batches: 256) consecutive cells of one
+//     mesh, for every mesh and every iteration, in one grid-stride launch
+//     (iterations need no ordering: the loops never read the dataset they
+//     increment); that kernel lives in atomic_batch.cu.
 // The reference has no counterpart (one mesh per process, one launch per
 // colour).
 #define FOT_ADAPTER_ALL 1

@@ -29,8 +29,10 @@ struct BatchDev {
 
 // Cells per tile of the atomic batch: the larger one spares look-ups, but a
 // batch that has less than 2.5 such tiles for each CTA is over sooner with the
-// smaller: AOS aggregated, one iteration, 1.3 tiles a CTA 16.0 us and 23.8 with
-// the larger, 2.1 26.1 and 28.9, 2.8 38.7 and 35.4, 6.8 98.2 and 88.4.
+// smaller: AOS aggregated, one iteration, 0.8 tiles a CTA 12.3 us and 13.1 with
+// the larger, 1.5 18.6 and 19.9, 2.2 26.0 and 26.9, 3.5 53.2 and 51.1, 7.1 104.5
+// and 98.7.  (Several iterations a call come to more tiles a CTA: with two, 0.8
+// 10.2 and 10.8, 1.5 16.7 and 16.5, 2.2 25.1 and 23.5 an iteration.)
 constexpr uint32_t kAtomicTile = 1024, kAtomicTileSmall = 256;
 
 // the atomic batch kernel for a set of loop kinds (atomic_batch.cu)

@@ -2,10 +2,10 @@
 //
 // (a) Global atomics (FOT_EXEC_ATOMIC) -- replaces the reference's
 //     global-colouring executor (problem.hpp:90-194, one launch and one
-//     cudaDeviceSynchronize per colour).  One thread per cell, mapping rows read as vectors, read sets gathered straight from
-//     HBM/L2, increments added with native atomics (f64 RED, AOS rows laid end
-//     to end across the warp first; one 16-byte f32x4 RED per row for the FP32
-//     loop).  With warp aggregation, runs of neighbouring lanes whose
+//     cudaDeviceSynchronize per colour).  One thread per cell, mapping rows
+//     read as vectors, read sets gathered straight from HBM/L2, increments
+//     added with native atomics (f64 RED, AOS rows laid end to end across the
+//     warp first; one 16-byte f32x4 RED per row for the FP32 loop).  With warp aggregation, runs of neighbouring lanes whose
 //     slot targets one point are summed in registers by a segmented shuffle
 //     tree before the run's first lane issues the atomics.
 //
@@ -109,8 +109,9 @@ struct Direct {
 // Read rows straight from global memory (problem layout AOS or SOA).  AOS rows
 // of a multiple of 4 doubles are fetched whole, one 32-byte load a sector,
 // where a cell's fit into registers; the user function then reads those:
-// coloured res_calc 1000^2, parts of 256, 48.7 -> 45.9 us.  miniAero's 56 values
-// do not (96^3 AOS 187 us, 257 fetched).
+// coloured res_calc 1000^2, parts of 256, 44.8 us an iteration, 48.1 without (the
+// atomic form 32.2 and 32.6).  miniAero's 56 values do not (96^3 AOS 187 us, 258
+// fetched).
 constexpr int kMostFetched = 16;
 template <class L, bool SOA> struct GlobalRows {
   using T = typename L::read_t;
@@ -239,11 +240,12 @@ template <class T> __device__ __forceinline__ void atomic_add(T *a, T v) { atomi
 // memory: reduction instruction i then covers elements [32 i, 32 i + 32) of
 // the rows laid end to end, so that neighbouring lanes fall into the same
 // 32-byte sectors of `out` (K = 4: 8 whole sectors an instruction).  Lane by
-// lane, component by component, each instruction touched 32 sectors, and the
-// L2's rate of atomic sectors bounded the loop: res_calc 1000^2 (4 doubles a
-// row) after RCM 97.3 us then, 45.1 us now; getacc 1024^2 108.0 and 45.5 us;
-// LULESH 96^3 (3 doubles) 92.5 and 49.6 us.  FP32 rows of 4 are one 16-byte
-// reduction and SOA data one run of addresses a component: neither needs it.
+// lane, component by component, each instruction would touch 32 sectors, and
+// the L2's rate of atomic sectors bound the loop: one iteration of res_calc
+// 1000^2 (4 doubles a row) after RCM 98.8 us so and 41.6 laid end to end (38.5 by
+// quads, below); getacc 1024^2 97.8 and 50.4 us; LULESH 96^3 (3 doubles) 92.2 and
+// 46.4 us.  FP32 rows of 4 are one 16-byte reduction and SOA data one run of
+// addresses a component: neither needs it.
 constexpr uint32_t kNoPoint = 0xFFFFFFFFu;
 template <int K>
 __device__ __forceinline__ void add_rows_f64(double *__restrict__ out, double *buf, uint32_t key,
@@ -272,11 +274,11 @@ __device__ __forceinline__ void add_rows_f64(double *__restrict__ out, double *b
 // of the quad's 4 rows.  Neighbouring rows with one key are then neighbouring
 // values of one lane: aggregation (AGG) sums those runs without a shuffle (runs
 // across quads stay separate reductions).  It spares half of the shared-memory
-// passes, and the L1's data path is what bounds loops that gather AOS rows
-// (res_calc 1000^2: 76% busy): with the 32-byte row loads, an iteration of 10
-// after RCM 36.2 -> 33.4 us, aggregated 36.3 -> 28.0.  A loop that gathers none
-// is better off with shared memory's fewer instructions: getacc 1024^2 45.2 us
-// so and 39.2 (aggregated 45.4 and 40.4).
+// passes, and the L1's data path is what bounds loops that gather AOS rows:
+// res_calc 1000^2, an iteration of 10 after RCM, 32.2 us so and 33.8 through
+// shared memory, aggregated 26.9 and 33.9.  A loop that gathers none is better
+// off with shared memory's fewer instructions: getacc 1024^2 44.6 us by quads
+// and 38.5 (aggregated 44.9 and 39.6).
 template <class L> constexpr bool by_quads() {
   return sizeof(typename L::out_t) == 8 && L::kOut == 4 && L::kNumRead > 0;
 }
@@ -324,9 +326,10 @@ __device__ __forceinline__ void add_rows4_f64(double *__restrict__ out, uint32_t
 // their points, so that equal keys lie side by side (2 edges, 3 faces of a
 // first cell); equal keys further apart stay separate reductions.  A warp
 // without runs pays one shuffle and one vote.  Grouping every lane with
-// __match_any_sync instead and gathering the group lane by lane cost more than
-// the reductions it saved: volna 1024^2 72.4 us, 42.5 us by runs; res_calc
-// 1000^2 SOA 49.0 and 41.3 us; LULESH 96^3 SOA 74.2 and 45.7 us (after RCM).
+// __match_any_sync instead and gathering the group lane by lane costs more than
+// the reductions it saves: one iteration of volna 1024^2 70.2 us, 42.6 us by runs;
+// res_calc 1000^2 SOA 38.4 and 30.8 us; LULESH 96^3 SOA 73.8 and 44.7 us (after
+// RCM).
 template <int K, class T>
 __device__ __forceinline__ bool sum_runs(uint32_t key, T (&inc)[K]) {
   const uint32_t lane = threadIdx.x & 31u;
@@ -433,31 +436,31 @@ template <class L> __device__ __forceinline__ void prefetch_cell(const LoopData 
 // when another reads it as a second point.  A CTA that lags behind loses
 // that, lags further, and the launch ends with idle SMs; at a phase's end the
 // CTAs fall into step again (the next phase's CTA starts where one finished
-// first), at the price of a CTA start per phase.  One round a CTA was always
-// slower than several (starts), and which loops drift was measured, R rounds a
-// phase against one phase for all: miniAero SOA 128^3 421 us (R = 4) and 585,
-// 120^3 342 and 352, but 96^3 177 and 172 (23 rounds in all: not split);
-// getacc 1024^2 43.4 and 45.1 (AOS), 1500x1600 SOA 88.7 and 101.1; volna 1024^2
-// 39.8 and 40.9 (R = 8); res_calc SOA without aggregation, fresh data, 1000^2
-// 37.3 and 38.9, 1200^2 51.5 and 55.1, 2000^2 133 and 149 (R = 6), aggregated 1200^2
-// 43.7 and 41.6, AOS 1000^2 34.0 and 33.3 (neither split); LULESH 96^3 44.2 and
-// 44.1, miniAero AOS 128^3 489 and 447 (never split).
+// first), at the price of a CTA start per phase.  Which loops drift was
+// measured, one iteration in phases of R rounds a CTA and in one phase for all:
+// miniAero SOA 128^3 422 us (R = 4) and 582, 120^3 341 and 351, but 96^3 175 and 170
+// (24 rounds in all: not split); getacc 1024^2 SOA 44.0 and 45.6 (R = 4; AOS 50 and
+// 50); volna 1024^2 SOA 41.8 and 43.0 (R = 8; AOS 38 and 38); res_calc SOA without
+// aggregation 1000^2 37.8 and 38.6, 1200^2 52.4 and 55.4, 2000^2 132 and 150 (R = 6),
+// aggregated 1200^2 45.9 and 43.4, AOS 1000^2 39.4 and 38.7 (neither split); LULESH
+// 96^3 45.6 and 44.4, miniAero AOS 128^3 486 and 452 (never split).
 //
 // The iterations of a call are one launch as well (no iteration reads what
 // another writes), each running through the mesh in the direction opposite to
-// the one before it, so that it starts on what is left in L2: 10 iterations of
-// res_calc 1000^2 SOA (152 MB each) 391 us as launches of their own, 329 us so
-// (after RCM, data not in L2 before the call); an iteration of 10, warm, of
-// LULESH 96^3 45.2 and 38.1 us, volna 1024^2 41.7 and 29.8, getacc 1024^2 45.9
-// and 34.2 (miniAero 128^3, 1.29 GB, gains its launch gaps only).
+// the one before it, so that it starts on what is left in L2.  An iteration of
+// 10, warm, as a launch of its own / in one launch in one direction / in
+// alternating directions: res_calc 1000^2 SOA 34.6 / 31.6 / 29.7 us, LULESH 96^3 SOA
+// 43.0 / 36.7 / 36.3, volna 1024^2 AOS 32.4 / 32.7 / 27.8, getacc 1024^2 AOS 41.4 /
+// 43.7 / 38.5 (the launches of their own alternate too; miniAero 128^3, 1.29 GB,
+// gains its launch gaps only).
 //
 // The grid starts while the one before it on the stream drains and waits for
 // its end (griddep_wait) before it touches memory, which hides the launch:
-// calls of one iteration one after the other, 64x48 res_calc 4.10 us and 3.4 us
-// (the host's rate), volna 300^2 6.2 and 4.4 us, LULESH 30^3 8.3 and 3.9.  It does
-// not let the next grid start before its own CTAs end (which all it could do
-// is wait): with an early griddepcontrol.launch_dependents LULESH 30^3 took 5.9
-// us, res_calc 200x210 4.2 (3.5 without), miniAero 80^3 118 (114).
+// calls of one iteration one after the other, with and without, 64x48 res_calc
+// 3.1 us (the host's rate) and 4.9, 200x210 3.5 and 6.2, volna 300^2 5.1 and 6.9,
+// LULESH 30^3 7.0 and 8.3.  It does not let the next grid start before its own
+// CTAs end (which all it could do is wait): with an early
+// griddepcontrol.launch_dependents LULESH 30^3 takes 11.6 us, the others the same.
 struct AtomicGrid {
   uint32_t tiles;     // of one iteration
   uint32_t resident;  // CTAs of a phase

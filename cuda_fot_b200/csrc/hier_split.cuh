@@ -23,17 +23,16 @@
 // next grid's tiles gather and compute (they only read datasets the loop never
 // writes) before they wait (griddepcontrol.wait) for this grid to complete and
 // only then write.  What a cell function writes to cell data is
-// held in a register until then (LULESH 45^3, 2 iterations 24.2 us waiting before
-// it computes, 22.8 so; 10 iterations 103 and 88; 30^3 68 and 56).
+// held in a register until then (an iteration of 10, waiting before it computes
+// and so: LULESH 45^3 10.6 and 9.1 us, 30^3 8.1 and 6.0).
 //
 // One CTA runs one tile (k_hier_dsplit); extra CTAs at the end of the grid do
 // the combine.  A warp-specialised persistent form that staged each tile's
 // read rows in shared memory (a record warp, a staging warp, two tiles in
-// flight) was slower on every loop, layout and ordering once this one summed
-// its contributions from lists, and is gone: parts of 256, staged and direct,
-// AOS: res_calc 1000^2 60.0 and 54.7 us, LULESH 96^3 113.9 and 87.2, volna 1024^2
-// 99.7 and 53.8, getacc 1024^2 77.2 and 52.6, miniAero 96^3 634 and 413;
-// LULESH 45^3 16.7 and 11.1.
+// flight) was slower on every loop, layout and partition once this one summed
+// its contributions from lists, and is gone (when it went, parts of 256, AOS,
+// staged and direct: res_calc 1000^2 60.0 and 54.7 us, 44.8 today; LULESH 96^3 113.9
+// and 87.2, 83.0 today; miniAero 96^3 634 and 413).
 #pragma once
 
 #include <cstdint>
@@ -140,8 +139,9 @@ __device__ __forceinline__ void comb_chunk(uint32_t n, uint32_t c, uint32_t part
 // thread with its K sums in registers: neighbouring lanes then write
 // neighbouring addresses of each component (SOA), or each a 16-byte row (FP32
 // AOS), and a point's contribution list is walked once.  Direct form, parts of
-// 256, by element and by point: res_calc 1000^2 AOS 63 and 77 us, getacc 1024^2
-// AOS 55 and 77; by point in SOA: res_calc 51 us, 63 by element.
+// 256, an iteration of 10, by element and by point: res_calc 1000^2 AOS 44.8 and
+// 62.1 us, getacc 1024^2 AOS 45.7 and 61.0; in SOA by point is the better one
+// (res_calc 51 us and 63 by element, when both were last there).
 template <class L, bool SOA> constexpr bool by_element() {
   return !SOA && sizeof(typename L::out_t) == 8;
 }
@@ -154,7 +154,7 @@ template <class L, bool SOA> constexpr bool by_row4() {
 // 16-byte load, read one row), component by component for SOA.  Rows of 4
 // doubles swap halves every 4 rows, so that the 16-byte stores of 8 lanes fall
 // into 8 different bank groups (2-way conflicts otherwise: res_calc 1000^2, parts
-// of 256, 51.8 us and 48.7, getacc 1024^2 49.0 and 46.2).
+// of 256, 47.7 us and 44.8 so, getacc 1024^2 47.5 and 45.7).
 template <class L, bool SOA, int T>
 __device__ __forceinline__ uint32_t inc_index(uint32_t ie, uint32_t k) {
   if constexpr (SOA) return k * (L::kDim * T) + ie;
@@ -284,10 +284,10 @@ __global__ void __launch_bounds__(T, dsplit_min_blocks<L, T>()) k_hier_dsplit(Lo
   // writes are not flushed yet) and gather what it has not written.
   if (P.ordered) griddep_wait();
   // Where the next grid has tiles that can gather and compute meanwhile, let it
-  // start; one that can only wait (the flush) takes longer when it starts
-  // early: res_calc 200x210, one iteration, 9.2 us and 6.5, LULESH 30^3 13.1 and
-  // 9.4; res_calc 1000^2, 10 iterations, 450 us with the early start and 465
-  // without.
+  // start (an iteration of 10 with and without: res_calc 1000^2 44.8 us and 46.3,
+  // 200x210 3.8 and 4.5, LULESH 45^3 9.1 and 10.7); the flush can only wait and
+  // gains nothing (one iteration, 200x210 7.4 us and 7.3 started early, LULESH
+  // 30^3 9.9 and 9.8).
   if (P.more) griddep_launch_dependents();
   const uint32_t n_tiles = P.tiles_on ? P.n_blocks : 0u;
   if (blockIdx.x >= n_tiles) {

@@ -92,9 +92,9 @@ int run_hier(const LoopData &d, const HierPlanDev &P, bool soa, uint32_t threads
     // before it lets the second start, because whatever precedes a call may
     // write the datasets that both read.  Iterations
     // alternate in direction, so that each starts on what the one before it
-    // left in L2 (parts of 256, 10 iterations, warm: res_calc 1000^2 AOS 54.7 us
-    // an iteration in one direction, 51.6 alternating; getacc 1024^2 52.6 and
-    // 49.3).
+    // left in L2 (parts of 256, 10 iterations, warm: res_calc 1000^2 AOS 48.5 us
+    // an iteration in one direction, 44.8 alternating; getacc 1024^2 49.8 and
+    // 45.7).
     const uint32_t iters = P.n_blocks ? P.total_tiles / P.n_blocks : 0;
     const uint32_t comb_ctas = (P.n_shared + threads - 1) / threads;  // a point a thread
     HierPlanDev Q = P;

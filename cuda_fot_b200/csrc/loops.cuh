@@ -55,11 +55,13 @@
 #define FOT_CAT(a, b) FOT_CAT2(a, b)
 #define FOT_LNS(name) FOT_CAT(name, FOT_NS_SUFFIX)
 // Resident CTAs per SM of the atomic executor, per loop (its register cap is
-// 65536 / (256 * this)); measured choices, overridable at build time.  After
-// RCM, AOS / SOA: res_calc 1000^2 5 CTAs 43.0 / 39.4 us, 4: 45.3 / 40.9, 6: 47.5 /
-// 45.5 (aggregated 43.4 / 36.4, 47.6 / 41.3, 47.6 / 36.2); mini_aero 96^3 3 CTAs (80
-// registers) 195 / 172 us, 2: 200 / 182 (4 CTAs spill too much: 321 / 285 with a
-// larger functor).
+// 65536 / (256 * this)); measured choices, overridable at build time.  An
+// iteration of 10 after RCM, AOS / SOA: res_calc 1000^2 5 CTAs 32.2 / 29.7 us, 4: 34.4
+// / 29.5, 6: 35.1 / 40.4 (aggregated 26.9 / 24.1, 29.2 / 25.6, 28.4 / 27.5); mini_aero
+// 96^3 3 CTAs (80 registers) 187 / 167 us, 2: 192 / 178, 4 (spills): 208 / 198; 128^3
+// 450 / 407, 472 / 436, 510 / 490.  A randomly numbered mesh wants 2 in SOA form (one
+// iteration, 80^3 899 us with 3 and 812, 96^3 2,451 and 2,090, 128^3 7,540 and 7,060),
+// which no size tells; ordered it takes a fifth of that time and less.
 #ifndef FOT_ATOMIC_MINB_RES_CALC
 #define FOT_ATOMIC_MINB_RES_CALC 5
 #endif
@@ -101,22 +103,27 @@
 #endif
 // atomic_carry: whether a warp of the atomic executor loads its next cells'
 // mapping rows while it computes the current ones.  An iteration of 10, warm,
-// without and with: LULESH 96^3 AOS / SOA 41.8 / 37.6 and 40.1 / 37.0 us; res_calc
-// 1000^2 SOA aggregated 27.1 and 25.5 (one iteration with its launch 41.0 and
-// 33.5), AOS 36.3 and 37.0: SOA only; volna 1024^2 AOS 29.8 and 28.7 (43.9 and
-// 42.8), aggregated 30.5 and 32.6: plain only; getacc 1024^2 SOA 34.3 and 35.8,
-// miniAero 128^3 SOA 417 and 417 (its rows are prefetched into L2): off.
+// without and with: LULESH 96^3 AOS 41.0 and 39.3 us, SOA 37.0 and 36.3; res_calc
+// 1000^2 SOA aggregated 25.4 and 24.1 (one iteration 33.0 and 30.8), AOS 32.2 and
+// 32.3: SOA only; volna 1024^2 one iteration 39.1 and 38.3, aggregated 42.6 and 41.0
+// but SOA 32.0 and 33.2 of 10: plain only; getacc 1024^2 SOA 33.0 and 34.1,
+// miniAero 128^3 SOA 414 and 418: off.
 // kDirectRegCap of the adapters below: registers per thread that the direct split
 // write-back kernel is held to; its tiles wait for memory at every step, so
-// that the CTAs an SM holds decide.  Parts of 256, AOS / SOA, by cap: res_calc
-// 1000^2 40: 54.7 / 49.7 us, 48: 59.5 / 50.6, 56: 65.6 / 57.1; volna 1024^2 32: 53.8 / 64.3,
-// 40: 64.7 / 82.1, 24: 65.9 / 82.7 (spills); parts of 128: LULESH 96^3 80: 92.7 /
-// 88.2, 72: 109 / 108 (spills), 96: 95.4 / 89.4; getacc 1024^2 56: 49.6 / 47.3, 48: 59.0 /
-// 53.2, 64: 53.3 / 49.6; miniAero hardly moves between 84 and 128.
+// that the CTAs an SM holds decide.  An iteration of 10, parts of 256, AOS / SOA,
+// by cap: res_calc 1000^2 40: 44.8 / 46.4 us, 48: 48.2 / 46.3, 56: 54.6 / 52.1; volna
+// 1024^2 32: 47.6 / 56.4, 40: 58.0 / 72.7, 24: 58.5 / 73.0 (spills); LULESH 96^3 80: 83.0
+// / 80.3, 96: 96.7 / 91.0; parts of 128: LULESH 80: 88.7 / 86.2, 96: 91.3 / 86.2, 72: 104
+// / 105 (spills); getacc 1024^2 56: 44.1 / 43.9, 64: 47.2 / 45.1, 48: 53.4 / 49.5;
+// miniAero hardly moves between 84 and 128.  (LULESH with its cells in random
+// order wants 96: a tile then writes a thousand points, and the increments and
+// records of 6 CTAs leave no L1 -- 96^3, blocks of 128, 403 us with 80 and 273.)
 // Whether the atomic executor (SOA form) prefetches the next chunk's mapping
 // rows and direct data into L2 while it computes the current one (per loop;
 // measured choices, overridable at build time: on for mini_aero's 96-byte
-// face records, 2% faster after RCM; 2-11% slower for the other loops).
+// face records, where it gains nothing any more: one iteration after RCM
+// 96^3 170.7 us with it and 172.0, 128^3 423 and 422; 2-11% slower for the other
+// loops).
 #ifndef FOT_ATOMIC_PREFETCH_RES_CALC
 #define FOT_ATOMIC_PREFETCH_RES_CALC 0
 #endif

@@ -358,7 +358,8 @@ int fot_airfoil_destroy(fot_airfoil *a);
  * Hierarchical plans: one persistent launch over a (mesh, block) tile queue
  * ordered by block colour per mesh; each mesh's result is that of its own
  * plan.  Atomic plans (all with or all without warp aggregation): one launch
- * over tiles of 1,024 (small batches 256) cells of every mesh and every iteration.  A batch holds
+ * over tiles of 1,024 cells (small batches 256) of every mesh and every iteration
+ * (several launches where the smaller tiles of a call pass 2^32).  A batch holds
  * one executor kind, one layout, and one loop kind or res_calc with volna.
  * No counterpart in the reference (one mesh per process). */
 int fot_batch_create(fot_problem *const *problems, fot_plan *const *plans,
