@@ -465,6 +465,9 @@ int fot_plan_build(fot_problem *p, const fot_plan_desc *desc, fot_plan **out) {
     }
     rc = build_hier_plan(p, plan);
     if (rc == FOT_OK) {
+      if ((plan->variant & kVariantSplit) &&
+          plan->stats.avg_block_points * plan->n_blocks > (double)ops->scattered_points * p->n_cells)
+        plan->variant |= kVariantScattered;
       plan->threads = hier_threads(desc->block_size);
       ops->smem_layout(plan->cap[0], plan->cap[1], plan->variant, plan->rec_cap, plan->threads,
                        &plan->layout);

@@ -31,8 +31,10 @@ struct SmemLayout {
 // double-buffered staging, per-point gather of the increments), launched
 // with 64 threads more than `threads` for its two control warps; bit 2 = that
 // kernel with three tile-record slots (else two); bit 3 = split write-back
-// (hier_split.cuh, one launch per iteration, one CTA per tile).
-constexpr uint32_t kVariantStage = 1u, kVariantPipe = 2u, kVariantSlots3 = 4u, kVariantSplit = 8u;
+// (hier_split.cuh, one launch per iteration, one CTA per tile); bit 4 = that
+// kernel with the registers of scattered blocks (LoopOps::scattered_points).
+constexpr uint32_t kVariantStage = 1u, kVariantPipe = 2u, kVariantSlots3 = 4u, kVariantSplit = 8u,
+                   kVariantScattered = 16u;
 
 struct LoopOps {
   // launch `iterations` iterations of the atomic executor; resident: CTAs the
@@ -54,6 +56,8 @@ struct LoopOps {
   // points per block and tile records of at most rec_cap bytes
   void (*smem_layout)(uint32_t cap0, uint32_t cap1, uint32_t variant, uint32_t rec_cap,
                       uint32_t threads, SmemLayout *out);
+  // a plan's blocks are scattered if they write more points a cell than this
+  uint32_t scattered_points;
 };
 
 const LoopOps *loop_ops(int loop);

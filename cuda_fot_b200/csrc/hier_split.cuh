@@ -265,12 +265,14 @@ template <class L> struct HeldValue<L, true> {
   typename L::written_t value;
 };
 
-template <class L, int T> constexpr int dsplit_min_blocks() {
-  return (65536 / (T * L::kDirectRegCap)) > 0 ? 65536 / (T * L::kDirectRegCap) : 1;
+// CAP: registers per thread (L::kDirectRegCap, or of plans with scattered
+// blocks L::kScatteredRegCap).
+constexpr int dsplit_min_blocks(int threads, int cap) {
+  return 65536 / (threads * cap) > 0 ? 65536 / (threads * cap) : 1;
 }
 
-template <class L, bool SOA, int T>
-__global__ void __launch_bounds__(T, dsplit_min_blocks<L, T>()) k_hier_dsplit(LoopData d, HierPlanDev P) {
+template <class L, bool SOA, int T, int CAP>
+__global__ void __launch_bounds__(T, dsplit_min_blocks(T, CAP)) k_hier_dsplit(LoopData d, HierPlanDev P) {
   using out_t = typename L::out_t;
   constexpr int D = L::kDim, K = L::kOut;
   extern __shared__ __align__(128) unsigned char smem[];

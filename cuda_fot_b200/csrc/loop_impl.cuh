@@ -43,21 +43,27 @@ template <bool SOA, uint32_t SLOTS> const void *pipe_kernel(uint32_t threads) {
   return nullptr;
 }
 
-template <bool SOA> const void *dsplit_kernel(uint32_t threads) {
+template <bool SOA, int CAP> const void *dsplit_kernel(uint32_t threads) {
   switch (threads) {
-  case 128: return reinterpret_cast<const void *>(&k_hier_dsplit<L, SOA, 128>);
-  case 256: return reinterpret_cast<const void *>(&k_hier_dsplit<L, SOA, 256>);
-  case 512: return reinterpret_cast<const void *>(&k_hier_dsplit<L, SOA, 512>);
+  case 128: return reinterpret_cast<const void *>(&k_hier_dsplit<L, SOA, 128, CAP>);
+  case 256: return reinterpret_cast<const void *>(&k_hier_dsplit<L, SOA, 256, CAP>);
+  // of so many threads an SM holds one CTA with either cap
+  case 512: return reinterpret_cast<const void *>(&k_hier_dsplit<L, SOA, 512, L::kDirectRegCap>);
   }
   return nullptr;
 }
 
 // variant: kVariantStage (staged reads), kVariantPipe (pipelined kernel),
-// kVariantSplit (split write-back kernel)
+// kVariantSplit (split write-back kernel), kVariantScattered (of scattered blocks)
 const void *kernel_for(int exec, bool soa, uint32_t threads, uint32_t variant) {
   if (exec == FOT_EXEC_ATOMIC) return nullptr;
-  if (exec == FOT_EXEC_HIER && (variant & kVariantSplit))
-    return soa ? dsplit_kernel<true>(threads) : dsplit_kernel<false>(threads);
+  if (exec == FOT_EXEC_HIER && (variant & kVariantSplit)) {
+    if (variant & kVariantScattered)
+      return soa ? dsplit_kernel<true, L::kScatteredRegCap>(threads)
+                 : dsplit_kernel<false, L::kScatteredRegCap>(threads);
+    return soa ? dsplit_kernel<true, L::kDirectRegCap>(threads)
+               : dsplit_kernel<false, L::kDirectRegCap>(threads);
+  }
   if (exec == FOT_EXEC_HIER && (variant & kVariantPipe)) {
     if (variant & kVariantSlots3) return soa ? pipe_kernel<true, 3>(threads) : pipe_kernel<false, 3>(threads);
     return soa ? pipe_kernel<true, 2>(threads) : pipe_kernel<false, 2>(threads);
@@ -203,5 +209,5 @@ void smem_layout(uint32_t cap0, uint32_t cap1, uint32_t variant, uint32_t rec_ca
 extern const LoopOps FOT_OPS_NAME;
 const LoopOps FOT_OPS_NAME = {FOT_CAT(atomic_run_, FOT_ADAPTER_NS), FOT_ADAPTER_NS::run_hier,
                               FOT_ADAPTER_NS::run_hier_colour, FOT_ADAPTER_NS::occupancy,
-                              FOT_ADAPTER_NS::smem_layout};
+                              FOT_ADAPTER_NS::smem_layout, FOT_ADAPTER_NS::L::kScatteredPoints};
 } // namespace fot

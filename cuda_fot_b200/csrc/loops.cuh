@@ -115,9 +115,15 @@
 // 1024^2 32: 47.6 / 56.4, 40: 58.0 / 72.7, 24: 58.5 / 73.0 (spills); LULESH 96^3 80: 83.0
 // / 80.3, 96: 96.7 / 91.0; parts of 128: LULESH 80: 88.7 / 86.2, 96: 91.3 / 86.2, 72: 104
 // / 105 (spills); getacc 1024^2 56: 44.1 / 43.9, 64: 47.2 / 45.1, 48: 53.4 / 49.5;
-// miniAero hardly moves between 84 and 128.  (LULESH with its cells in random
-// order wants 96: a tile then writes a thousand points, and the increments and
-// records of 6 CTAs leave no L1 -- 96^3, blocks of 128, 403 us with 80 and 273.)
+// miniAero hardly moves between 84 and 128.
+// kScatteredRegCap: the cap of plans whose blocks write more than kScatteredPoints
+// points a cell, where it differs.  LULESH blocks of neighbouring elements write
+// 1.8 to 3.6 points a cell (96 to 20^3: every ordering, and nodes numbered at
+// random), blocks of elements in random order 4.4 to 4.7: the increments and
+// records of 6 CTAs of those leave next to no L1, 5 have room.  An iteration of 5
+// with a cap of 80 and of 96: 96^3 405 and 276 us (blocks of 128), 415 and 262 (256),
+// 45^3 28.0 and 18.5, 20^3 9.2 and 8.5; below the line 96 is 0 to 11% faster with
+// random nodes but 0 to 25% slower with ordered ones.
 // Whether the atomic executor (SOA form) prefetches the next chunk's mapping
 // rows and direct data into L2 while it computes the current one (per loop;
 // measured choices, overridable at build time: on for mini_aero's 96-byte
@@ -166,6 +172,8 @@ struct Loop {
   static constexpr int kRegCap = 64; // registers per thread the tile kernels are held to
   // registers per thread of the direct split write-back kernel
   static constexpr int kDirectRegCap = 40;
+  static constexpr int kScatteredRegCap = kDirectRegCap;
+  static constexpr int kScatteredPoints = kDim;
   // resident 256-thread CTAs per SM the atomic executor is compiled for
   static constexpr int kAtomicMinBlocks = FOT_ATOMIC_MINB_RES_CALC;
   // the atomic executor prefetches the next chunk into L2
@@ -216,6 +224,8 @@ struct Loop {
   static constexpr int kRegCap = 128; // registers per thread the tile kernels are held to
   // registers per thread of the direct split write-back kernel
   static constexpr int kDirectRegCap = kRegCap;
+  static constexpr int kScatteredRegCap = kDirectRegCap;
+  static constexpr int kScatteredPoints = kDim;
   // resident 256-thread CTAs per SM the atomic executor is compiled for
   static constexpr int kAtomicMinBlocks = FOT_ATOMIC_MINB_MINI_AERO;
   // the atomic executor prefetches the next chunk into L2
@@ -276,6 +286,9 @@ struct Loop {
   static constexpr int kRegCap = 96; // registers per thread the tile kernels are held to
   // registers per thread of the direct split write-back kernel
   static constexpr int kDirectRegCap = 80;
+  // of plans whose blocks write more than kScatteredPoints points a cell
+  static constexpr int kScatteredRegCap = 96;
+  static constexpr int kScatteredPoints = 4;
   // resident 256-thread CTAs per SM the atomic executor is compiled for
   static constexpr int kAtomicMinBlocks = FOT_ATOMIC_MINB_LULESH;
   // the atomic executor prefetches the next chunk into L2
@@ -336,6 +349,8 @@ struct Loop {
   static constexpr int kRegCap = 64; // registers per thread the tile kernels are held to
   // registers per thread of the direct split write-back kernel
   static constexpr int kDirectRegCap = 32;
+  static constexpr int kScatteredRegCap = kDirectRegCap;
+  static constexpr int kScatteredPoints = kDim;
   // resident 256-thread CTAs per SM the atomic executor is compiled for
   static constexpr int kAtomicMinBlocks = FOT_ATOMIC_MINB_VOLNA;
   // the atomic executor prefetches the next chunk into L2
@@ -388,6 +403,8 @@ struct Loop {
   static constexpr int kRegCap = 96; // registers per thread the tile kernels are held to
   // registers per thread of the direct split write-back kernel
   static constexpr int kDirectRegCap = 56;
+  static constexpr int kScatteredRegCap = kDirectRegCap;
+  static constexpr int kScatteredPoints = kDim;
   // resident 256-thread CTAs per SM the atomic executor is compiled for
   static constexpr int kAtomicMinBlocks = FOT_ATOMIC_MINB_GETACC;
   // the atomic executor prefetches the next chunk into L2
