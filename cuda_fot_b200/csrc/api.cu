@@ -202,7 +202,8 @@ static int enqueue_plan(fot_problem *p, fot_plan *plan, uint32_t iterations, boo
     return fail(FOT_ERR_STATE, "plan is stale: the problem's point layout changed after the plan was built");
   if (plan->desc.exec == FOT_EXEC_ATOMIC) {
     const bool agg = !(plan->desc.flags & FOT_PLAN_NO_AGGREGATE);
-    return ops->run_atomic(d, soa, agg, (uint32_t)(plan->per_sm * sms), iterations, backwards, st);
+    return ops->run_atomic(d, soa, agg, plan->variant & kVariantScattered, (uint32_t)(plan->per_sm * sms),
+                           iterations, backwards, st);
   }
   if (plan->version != p->version)
     return fail(FOT_ERR_STATE, "plan is stale: the problem was reordered after the plan was built");
@@ -449,7 +450,15 @@ int fot_plan_build(fot_problem *p, const fot_plan_desc *desc, fot_plan **out) {
   if (desc->exec == FOT_EXEC_ATOMIC) {
     plan->threads = 256;
     const uint32_t agg = (desc->flags & FOT_PLAN_NO_AGGREGATE) ? 0u : 1u;
-    rc = ops->occupancy(FOT_EXEC_ATOMIC, p->layout == FOT_SOA, 256, agg, 0, &plan->per_sm);
+    // as the mesh is ordered now (an atomic plan outlives a reordering; its
+    // results do not depend on the form)
+    if (p->layout == FOT_SOA && ops->scattered_sectors < 32) {
+      double sectors = 0;
+      rc = sectors_per_warp(p, p->info.point_type_size[1], &sectors);
+      if (rc == FOT_OK && sectors > ops->scattered_sectors) plan->variant = kVariantScattered;
+    }
+    if (rc == FOT_OK)
+      rc = ops->occupancy(FOT_EXEC_ATOMIC, p->layout == FOT_SOA, 256, agg | plan->variant, 0, &plan->per_sm);
   } else if (desc->exec == FOT_EXEC_HIER || desc->exec == FOT_EXEC_HIER_LAUNCH) {
     // Persistent executor (blocks of at most 512 cells): the split write-back
     // kernel by default, the pipelined kernel with per-block completion

@@ -32,14 +32,16 @@ struct SmemLayout {
 // with 64 threads more than `threads` for its two control warps; bit 2 = that
 // kernel with three tile-record slots (else two); bit 3 = split write-back
 // (hier_split.cuh, one launch per iteration, one CTA per tile); bit 4 = that
-// kernel with the registers of scattered blocks (LoopOps::scattered_points).
+// kernel with the registers of scattered blocks (LoopOps::scattered_points);
+// atomic plans: the form of scattered rows.
 constexpr uint32_t kVariantStage = 1u, kVariantPipe = 2u, kVariantSlots3 = 4u, kVariantSplit = 8u,
                    kVariantScattered = 16u;
 
 struct LoopOps {
-  // launch `iterations` iterations of the atomic executor; resident: CTAs the
-  // GPU holds at once; backwards: the first one runs last tile to first
-  int (*run_atomic)(const LoopData &d, bool soa, bool aggregate, uint32_t resident,
+  // launch `iterations` iterations of the atomic executor; scattered: the form
+  // of scattered rows, where the loop has one; resident: CTAs the GPU holds at
+  // once; backwards: the first one runs last tile to first
+  int (*run_atomic)(const LoopData &d, bool soa, bool aggregate, bool scattered, uint32_t resident,
                     uint32_t iterations, bool backwards, cudaStream_t st);
   // persistent hierarchical launch over P.total_tiles tiles (backwards: split
   // write-back kernel only)
@@ -58,6 +60,9 @@ struct LoopOps {
                       uint32_t threads, SmemLayout *out);
   // a plan's blocks are scattered if they write more points a cell than this
   uint32_t scattered_points;
+  // a problem's rows are scattered if 32 neighbouring cells' fall into more
+  // sectors of a component than this (32: the loop has no form of its own)
+  uint32_t scattered_sectors;
 };
 
 const LoopOps *loop_ops(int loop);
@@ -76,6 +81,9 @@ inline int set_class(int loop, uint32_t k) {
 }
 
 int device_sm_count();
+// Mean number of 32-byte sectors that a slot's rows of 32 neighbouring cells
+// fall into, a component of SOA data of `size` bytes a value (features.cu).
+int sectors_per_warp(const fot_problem *p, uint32_t size, double *out);
 
 } // namespace fot
 

@@ -473,8 +473,12 @@ struct AtomicGrid {
 // cells it will take next, so that their mapping rows and direct data come
 // from L2 then; with L::atomic_carry it loads their mapping rows into
 // registers, a memory latency ahead of the rows that they point to.
-template <class L, bool SOA, bool AGG>
-__global__ void __launch_bounds__(256, L::kAtomicMinBlocks) k_atomic(LoopData d, AtomicGrid g) {
+// SCATTERED: the form of problems whose rows are scattered (loops.cuh).
+template <class L, bool SCATTERED> constexpr int atomic_min_blocks() {
+  return SCATTERED ? L::kAtomicScatteredMinBlocks : L::kAtomicMinBlocks;
+}
+template <class L, bool SOA, bool AGG, bool SCATTERED>
+__global__ void __launch_bounds__(256, (atomic_min_blocks<L, SCATTERED>())) k_atomic(LoopData d, AtomicGrid g) {
   const uint32_t in_tile = threadIdx.x & ~31u, lane = threadIdx.x & 31u;
   griddep_wait();
   const uint32_t it = blockIdx.x / g.ctas, b = blockIdx.x - it * g.ctas;
@@ -489,7 +493,7 @@ __global__ void __launch_bounds__(256, L::kAtomicMinBlocks) k_atomic(LoopData d,
     const uint32_t n = t + g.resident;
     const uint32_t next = (back ? g.tiles - 1u - n : n) * 256u + in_tile + lane;
     const bool more = r + 1 < g.rounds && n < g.tiles;
-    if constexpr (L::kAtomicPrefetch && SOA) {
+    if constexpr (L::kAtomicPrefetch && SOA && !SCATTERED) {
       if (more && next < d.n_cells) prefetch_cell<L>(d, next);
     }
     if constexpr (kCarry) {

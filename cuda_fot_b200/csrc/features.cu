@@ -48,6 +48,22 @@ __global__ void k_row_span(const uint32_t *__restrict__ map, uint32_t n, int D,
   }
 }
 
+// Sectors of a component (points / per_sector) that each slot's rows of 32
+// neighbouring cells fall into, summed over slots and the warps of the grid,
+// whose groups of cells are spread evenly over the mesh.
+__global__ void k_warp_sectors(const uint32_t *__restrict__ map, uint32_t n, int D, uint32_t per_sector,
+                               unsigned int *sum) {
+  const uint32_t warps = gridDim.x * (blockDim.x / 32), warp = blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32;
+  const uint32_t lane = threadIdx.x & 31u, groups = (n + 31) / 32;
+  const uint32_t c = min((uint32_t)((uint64_t)groups * warp / warps) * 32 + lane, n - 1);
+  unsigned int total = 0;
+  for (int q = 0; q < D; ++q) {
+    const unsigned same = __match_any_sync(0xFFFFFFFFu, map[(size_t)c * D + q] / per_sector);
+    total += __popc(__ballot_sync(0xFFFFFFFFu, __ffs(same) - 1 == (int)lane));
+  }
+  if (lane == 0) atomicAdd(sum, total);
+}
+
 __global__ void k_point_degree(const uint32_t *__restrict__ map, size_t ne, uint32_t *deg) {
   for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < ne; e += (size_t)gridDim.x * blockDim.x)
     atomicAdd(&deg[map[e]], 1u);
@@ -207,6 +223,22 @@ int count_distinct(DevBuf &keys, size_t n_keys, uint64_t *count) {
 }
 
 } // namespace
+int sectors_per_warp(const fot_problem *p, uint32_t size, double *out) {
+  const uint32_t ctas = 32, warps = ctas * 8;
+  const int D = (int)p->mesh_dim();
+  // the thread's scratch: an allocation of its own would take longer than the rest
+  void *sum = nullptr;
+  FOT_TRY(cub_scratch(sizeof(unsigned int), &sum));
+  FOT_CUDA(cudaMemset(sum, 0, sizeof(unsigned int)));
+  k_warp_sectors<<<ctas, 256>>>(p->map[0].as<uint32_t>(), p->n_cells, D, 32 / size,
+                                static_cast<unsigned int *>(sum));
+  FOT_CUDA(cudaGetLastError());
+  unsigned int total = 0;
+  FOT_CUDA(cudaMemcpy(&total, sum, sizeof(total), cudaMemcpyDeviceToHost));
+  *out = (double)total / (warps * D);
+  return FOT_OK;
+}
+
 } // namespace fot
 
 using namespace fot;

@@ -21,11 +21,19 @@ namespace {
 
 using LA = FOT_LNS(FOT_ADAPTER_NS)::Loop;
 
+// whether the loop has a form of its own for scattered rows
+template <bool SOA> constexpr bool has_scattered() {
+  return SOA && LA::kAtomicScatteredMinBlocks != LA::kAtomicMinBlocks;
+}
+
 // `iterations` iterations in one launch (more only where the grid would grow
 // past 2^30 CTAs).
-template <bool SOA, bool AGG>
-int launch_atomic(const LoopData &d, uint32_t resident, uint32_t iterations, bool backwards,
-                  cudaStream_t st) {
+template <bool SOA, bool AGG, bool SCATTERED = false>
+int launch_atomic(const LoopData &d, bool scattered, uint32_t resident, uint32_t iterations,
+                  bool backwards, cudaStream_t st) {
+  if constexpr (!SCATTERED && has_scattered<SOA>()) {
+    if (scattered) return launch_atomic<SOA, AGG, true>(d, true, resident, iterations, backwards, st);
+  }
   AtomicGrid g;
   g.flip = backwards;
   g.tiles = (d.n_cells + 255u) / 256u;
@@ -39,30 +47,34 @@ int launch_atomic(const LoopData &d, uint32_t resident, uint32_t iterations, boo
   while (iterations) {
     const uint32_t now = std::min(iterations, most);
     Chained c(dim3(g.ctas * now), dim3(256), 0, st);
-    FOT_CUDA(cudaLaunchKernelEx(&c.cfg, k_atomic<LA, SOA, AGG>, d, g));
+    FOT_CUDA(cudaLaunchKernelEx(&c.cfg, k_atomic<LA, SOA, AGG, SCATTERED>, d, g));
     iterations -= now;
     g.flip += now;
   }
   return FOT_OK;
 }
 
-template <bool SOA, bool AGG> const void *atomic_kernel() {
-  return reinterpret_cast<const void *>(&k_atomic<LA, SOA, AGG>);
+template <bool SOA, bool AGG> const void *atomic_kernel(bool scattered) {
+  if constexpr (has_scattered<SOA>()) {
+    if (scattered) return reinterpret_cast<const void *>(&k_atomic<LA, SOA, AGG, true>);
+  }
+  return reinterpret_cast<const void *>(&k_atomic<LA, SOA, AGG, false>);
 }
 
 } // namespace
 
-int FOT_CAT(atomic_run_, FOT_ADAPTER_NS)(const LoopData &d, bool soa, bool agg, uint32_t resident,
-                                         uint32_t iterations, bool backwards, cudaStream_t st) {
-  if (soa) return agg ? launch_atomic<true, true>(d, resident, iterations, backwards, st)
-                      : launch_atomic<true, false>(d, resident, iterations, backwards, st);
-  return agg ? launch_atomic<false, true>(d, resident, iterations, backwards, st)
-             : launch_atomic<false, false>(d, resident, iterations, backwards, st);
+int FOT_CAT(atomic_run_, FOT_ADAPTER_NS)(const LoopData &d, bool soa, bool agg, bool scattered,
+                                         uint32_t resident, uint32_t iterations, bool backwards,
+                                         cudaStream_t st) {
+  if (soa) return agg ? launch_atomic<true, true>(d, scattered, resident, iterations, backwards, st)
+                      : launch_atomic<true, false>(d, scattered, resident, iterations, backwards, st);
+  return agg ? launch_atomic<false, true>(d, scattered, resident, iterations, backwards, st)
+             : launch_atomic<false, false>(d, scattered, resident, iterations, backwards, st);
 }
 
-int FOT_CAT(atomic_occupancy_, FOT_ADAPTER_NS)(bool soa, bool agg, int *per_sm) {
-  const void *k = soa ? (agg ? atomic_kernel<true, true>() : atomic_kernel<true, false>())
-                      : (agg ? atomic_kernel<false, true>() : atomic_kernel<false, false>());
+int FOT_CAT(atomic_occupancy_, FOT_ADAPTER_NS)(bool soa, bool agg, bool scattered, int *per_sm) {
+  const void *k = soa ? (agg ? atomic_kernel<true, true>(scattered) : atomic_kernel<true, false>(scattered))
+                      : (agg ? atomic_kernel<false, true>(scattered) : atomic_kernel<false, false>(scattered));
   FOT_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, k, 256, 0));
   return FOT_OK;
 }

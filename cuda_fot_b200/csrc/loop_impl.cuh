@@ -11,9 +11,10 @@
 namespace fot {
 
 // the atomic executor of this loop (atomic_*.cu, loop_atomic_impl.cuh)
-int FOT_CAT(atomic_run_, FOT_ADAPTER_NS)(const LoopData &d, bool soa, bool agg, uint32_t resident,
-                                         uint32_t iterations, bool backwards, cudaStream_t st);
-int FOT_CAT(atomic_occupancy_, FOT_ADAPTER_NS)(bool soa, bool agg, int *per_sm);
+int FOT_CAT(atomic_run_, FOT_ADAPTER_NS)(const LoopData &d, bool soa, bool agg, bool scattered,
+                                         uint32_t resident, uint32_t iterations, bool backwards,
+                                         cudaStream_t st);
+int FOT_CAT(atomic_occupancy_, FOT_ADAPTER_NS)(bool soa, bool agg, bool scattered, int *per_sm);
 
 namespace FOT_ADAPTER_NS {
 
@@ -135,9 +136,10 @@ int run_hier_colour(const LoopData &d, const HierPlanDev &P, bool soa, uint32_t 
 }
 
 int occupancy(int exec, bool soa, uint32_t threads, uint32_t variant, size_t smem, int *per_sm) {
-  // atomic plans: `variant` bit 0 set = warp aggregation
+  // atomic plans: `variant` bit 0 set = warp aggregation, kVariantScattered =
+  // scattered rows
   if (exec == FOT_EXEC_ATOMIC)
-    return FOT_CAT(atomic_occupancy_, FOT_ADAPTER_NS)(soa, variant & 1u, per_sm);
+    return FOT_CAT(atomic_occupancy_, FOT_ADAPTER_NS)(soa, variant & 1u, variant & kVariantScattered, per_sm);
   const void *k = kernel_for(exec, soa, threads, variant);
   if (!k) return fail(FOT_ERR_ARG, "no kernel for %u threads", threads);
   FOT_TRY(prepare(k, smem));
@@ -209,5 +211,8 @@ void smem_layout(uint32_t cap0, uint32_t cap1, uint32_t variant, uint32_t rec_ca
 extern const LoopOps FOT_OPS_NAME;
 const LoopOps FOT_OPS_NAME = {FOT_CAT(atomic_run_, FOT_ADAPTER_NS), FOT_ADAPTER_NS::run_hier,
                               FOT_ADAPTER_NS::run_hier_colour, FOT_ADAPTER_NS::occupancy,
-                              FOT_ADAPTER_NS::smem_layout, FOT_ADAPTER_NS::L::kScatteredPoints};
+                              FOT_ADAPTER_NS::smem_layout, FOT_ADAPTER_NS::L::kScatteredPoints,
+                              FOT_ADAPTER_NS::L::kAtomicScatteredMinBlocks != FOT_ADAPTER_NS::L::kAtomicMinBlocks
+                                  ? kScatteredSectors
+                                  : 32};
 } // namespace fot

@@ -59,14 +59,26 @@
 // iteration of 10 after RCM, AOS / SOA: res_calc 1000^2 5 CTAs 32.2 / 29.7 us, 4: 34.4
 // / 29.5, 6: 35.1 / 40.4 (aggregated 26.9 / 24.1, 29.2 / 25.6, 28.4 / 27.5); mini_aero
 // 96^3 3 CTAs (80 registers) 187 / 167 us, 2: 192 / 178, 4 (spills): 208 / 198; 128^3
-// 450 / 407, 472 / 436, 510 / 490.  A randomly numbered mesh wants 2 in SOA form (one
-// iteration, 80^3 899 us with 3 and 812, 96^3 2,451 and 2,090, 128^3 7,540 and 7,060),
-// which no size tells; ordered it takes a fifth of that time and less.
+// 450 / 407, 472 / 436, 510 / 490.
+// FOT_ATOMIC_SCATTERED_MINB_*: the same, in SOA form, of problems whose rows are
+// scattered: 32 neighbouring cells' rows fall into more than
+// kScatteredSectors sectors of a component, of 32 at most.  Every gather then
+// misses, and more warps in flight cost more of L2 than they hide.  miniAero,
+// one iteration plain with 3 CTAs and with 2 (which do not prefetch into L2
+// either, 0 to 5% there): randomly numbered, 32 sectors, 72^3 419 us and 352, 80^3
+// 884 and 787, 96^3 2,429 and 2,089, 128^3 7,480 and 7,030; after ORDER_RANDOM,
+// which sorts the cells, 19 sectors, 80^3 393 and 350, 96^3 1,181 and 956, 128^3
+// 3,808 and 3,620, 40^3 35.3 and 33.5.  Meshes in any useful order have 4 to 12:
+// RCM (7 to 10) 96^3 169 and 195, in parts of 128 (11) 222 and 233, as generated
+// without permutation (8) 217 and 214.
 #ifndef FOT_ATOMIC_MINB_RES_CALC
 #define FOT_ATOMIC_MINB_RES_CALC 5
 #endif
 #ifndef FOT_ATOMIC_MINB_MINI_AERO
 #define FOT_ATOMIC_MINB_MINI_AERO 3
+#endif
+#ifndef FOT_ATOMIC_SCATTERED_MINB_MINI_AERO
+#define FOT_ATOMIC_SCATTERED_MINB_MINI_AERO 2
 #endif
 #ifndef FOT_ATOMIC_MINB_LULESH
 #define FOT_ATOMIC_MINB_LULESH 2
@@ -151,6 +163,8 @@
 
 namespace fot {
 
+constexpr int kScatteredSectors = 16;
+
 // --------------------------------------------------------------------------
 // res_calc: edge -> 2 cells; reads x through the edge->node mapping and q,
 // adt through the edge->cell mapping (res_calc.hpp:29-89).
@@ -176,6 +190,7 @@ struct Loop {
   static constexpr int kScatteredPoints = kDim;
   // resident 256-thread CTAs per SM the atomic executor is compiled for
   static constexpr int kAtomicMinBlocks = FOT_ATOMIC_MINB_RES_CALC;
+  static constexpr int kAtomicScatteredMinBlocks = kAtomicMinBlocks;
   // the atomic executor prefetches the next chunk into L2
   static constexpr bool kAtomicPrefetch = FOT_ATOMIC_PREFETCH_RES_CALC;
   // it loads the next mapping rows ahead
@@ -228,6 +243,8 @@ struct Loop {
   static constexpr int kScatteredPoints = kDim;
   // resident 256-thread CTAs per SM the atomic executor is compiled for
   static constexpr int kAtomicMinBlocks = FOT_ATOMIC_MINB_MINI_AERO;
+  // the same of problems whose rows are scattered (SOA form)
+  static constexpr int kAtomicScatteredMinBlocks = FOT_ATOMIC_SCATTERED_MINB_MINI_AERO;
   // the atomic executor prefetches the next chunk into L2
   static constexpr bool kAtomicPrefetch = FOT_ATOMIC_PREFETCH_MINI_AERO;
   // it loads the next mapping rows ahead
@@ -291,6 +308,7 @@ struct Loop {
   static constexpr int kScatteredPoints = 4;
   // resident 256-thread CTAs per SM the atomic executor is compiled for
   static constexpr int kAtomicMinBlocks = FOT_ATOMIC_MINB_LULESH;
+  static constexpr int kAtomicScatteredMinBlocks = kAtomicMinBlocks;
   // the atomic executor prefetches the next chunk into L2
   static constexpr bool kAtomicPrefetch = FOT_ATOMIC_PREFETCH_LULESH;
   // it loads the next mapping rows ahead
@@ -353,6 +371,7 @@ struct Loop {
   static constexpr int kScatteredPoints = kDim;
   // resident 256-thread CTAs per SM the atomic executor is compiled for
   static constexpr int kAtomicMinBlocks = FOT_ATOMIC_MINB_VOLNA;
+  static constexpr int kAtomicScatteredMinBlocks = kAtomicMinBlocks;
   // the atomic executor prefetches the next chunk into L2
   static constexpr bool kAtomicPrefetch = FOT_ATOMIC_PREFETCH_VOLNA;
   // it loads the next mapping rows ahead
@@ -407,6 +426,7 @@ struct Loop {
   static constexpr int kScatteredPoints = kDim;
   // resident 256-thread CTAs per SM the atomic executor is compiled for
   static constexpr int kAtomicMinBlocks = FOT_ATOMIC_MINB_GETACC;
+  static constexpr int kAtomicScatteredMinBlocks = kAtomicMinBlocks;
   // the atomic executor prefetches the next chunk into L2
   static constexpr bool kAtomicPrefetch = FOT_ATOMIC_PREFETCH_GETACC;
   // it loads the next mapping rows ahead
