@@ -3,6 +3,8 @@
 //   fot_mesh_features      the spread of mapping 0's rows in the current
 //                          numbering (largest and mean max - min of a cell's
 //                          points) and the histogram of point degrees;
+//   sectors_per_warp       how far apart neighbouring cells' rows lie (which form
+//                          of the atomic executor a plan takes)
 //   fot_sector_count       the reference's sector model
 //   fot_plan_sector_count  (countCacheLinesForBlock, problem.hpp:654-672, as
 //                          loopGPUCellCentred / loopGPUHierarchical use it,
